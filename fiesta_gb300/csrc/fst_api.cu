@@ -26,7 +26,10 @@ DivC make_div(double d) {
   q.d = d;
   int e = 0;
   double m = std::frexp(d, &e);
-  q.inv = (d > 0.0 && m == 0.5 && std::isfinite(1.0 / d)) ? 1.0 / d : 0.0;
+  // (|k| <= 1000: scale2's range; a wilder spacing takes the division)
+  q.inv = (d > 0.0 && m == 0.5 && e > -1000 && e < 1000) ? 1.0 / d : 0.0;
+  q.k = 1 - e;  // d = 2^(e-1)
+  q.r = fst64::recip_of(d);
   return q;
 }
 
@@ -164,13 +167,13 @@ void setup_phys(const fst_config& cf, const Geo& g, Phys& P) {
   P.d4x = make_div(4 * P.dx);
   P.d4y = make_div(4 * P.dy);
   P.d4z = make_div(4 * P.dz);
-  P.d12x = 12.0 * P.dx;
-  P.d12y = 12.0 * P.dy;
-  P.d12z = 12.0 * P.dz;
-  P.d12pz = 12.0 * P.dy;
-  P.r12x = 1.0 / P.d12x;
-  P.r12y = 1.0 / P.d12y;
-  P.r12pz = 1.0 / P.d12pz;
+  P.d12x = make_div(12.0 * P.dx);
+  P.d12y = make_div(12.0 * P.dy);
+  P.d12z = make_div(12.0 * P.dz);
+  P.d12pz = make_div(12.0 * P.dy);
+  P.r12x = 1.0 / P.d12x.d;
+  P.r12y = 1.0 / P.d12y.d;
+  P.r12pz = 1.0 / P.d12pz.d;
   P.dt = cf.dt;
   P.hdt = 0.5f * cf.dt;
   P.kap = cf.kap;
@@ -190,9 +193,9 @@ void setup_phys(const fst_config& cf, const Geo& g, Phys& P) {
   P.rd_f[0] = (float)(1.0 / P.dx);
   P.rd_f[1] = (float)(1.0 / P.dy);
   P.rd_f[2] = (float)(1.0 / P.dz);
-  P.r12_f[0] = (float)(1.0 / P.d12x);
-  P.r12_f[1] = (float)(1.0 / P.d12y);
-  P.r12_f[2] = (float)(1.0 / P.d12z);
+  P.r12_f[0] = (float)(1.0 / P.d12x.d);
+  P.r12_f[1] = (float)(1.0 / P.d12y.d);
+  P.r12_f[2] = (float)(1.0 / P.d12z.d);
   P.dxmag_f = (float)P.dxmag;
   P.dxmag2_f = (float)P.dxmag2;
   P.eps_f = (float)P.eps;

@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include "../../include/fst.h"
+#include "fst_fp64.cuh"
 
 #define FST_MAXV (4 + FST_MAX_SPECIES + 5)
 
@@ -18,14 +19,17 @@ struct Geo {
   long long sy, sz, sv;
 };
 
-// Division by a run-time constant d.  When d is a power of two, a/d equals
-// a*(1/d) exactly for every a (both are the correctly rounded a*2^-k), so the
-// multiply is used; otherwise the IEEE division.  Results are bit-identical
-// to a/d either way.
+// Division by a run-time constant d, on the integer pipes (fst_fp64.cuh).
+// When d is a power of two, a/d equals a*(1/d) exactly for every a (both are
+// the correctly rounded a*2^k) and the exponent is shifted; otherwise the
+// integer division with d's reciprocal prepared on the host.  Results are
+// bit-identical to a/d either way.
 struct DivC {
   double d, inv;  // inv = 1/d if d is a power of two, else 0
+  int k;          // inv = 2^k
+  fst64::Recip r;
   __device__ __forceinline__ double operator()(double a) const {
-    return inv != 0.0 ? a * inv : a / d;
+    return inv != 0.0 ? fst64::scale2(a, k, inv) : fst64::div_by(a, r);
   }
 };
 
@@ -43,8 +47,8 @@ struct Phys {
   double dx, dy, dz;
   DivC ddx, ddy, ddz;     // x/dx, x/dy, x/dz
   DivC d4x, d4y, d4z;     // x/(4*dx) ... (viscous and C-equation tangential terms)
-  double d12x, d12y, d12z;  // 12.0*dx, 12.0*dy, 12.0*dz (4th-order derivatives)
-  double d12pz;           // 12.0*cd(2): the reference's dz = cd(2) in presgrad3D
+  DivC d12x, d12y, d12z;  // x/(12.0*dx) ... (4th-order derivatives)
+  DivC d12pz;             // x/(12.0*cd(2)): the reference's dz = cd(2) in presgrad3D
   double r12x, r12y, r12pz;  // their reciprocals (mixed path)
   double dt, hdt;         // dt and 0.5f*dt
   double kap, eps, alpha, g, rho_ref;

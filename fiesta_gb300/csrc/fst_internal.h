@@ -230,7 +230,7 @@ int fst_mixed_upload(const Geo& g, const Phys& P, MixedBufs& b, const double* Uh
 struct NoiseGraph {
   cudaStream_t cap = nullptr;  // capture stream (the caller's may be the legacy stream)
   cudaGraphExec_t exec = nullptr;
-  unsigned char sig[128] = {};
+  unsigned char sig[160] = {};
   int launches = 0;
 };
 void fst_noise_graph_release(NoiseGraph& ng);

@@ -30,6 +30,7 @@
 #include "fst_internal.h"
 
 namespace {
+using fst64::div_by;
 
 constexpr int T3 = 8;   // 3D tile edge (cells)
 constexpr int T2 = 32;  // 2D tile edge
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(256) k_noise_detect(Geo g, const double* __res
 struct RemoveArgs {
   int nvars, vars[3];
   double eta, dx, dy, dz;
+  fst64::Recip rx, ry, rz;  // divisors: dx^2, dy^2, dz^2 (2D: dx, dy)
   long long safe;
 };
 
@@ -369,9 +371,10 @@ __global__ void __launch_bounds__(R3, 3) k_noise_remove3(Geo g, double* __restri
         double (*sv3)[E][E] = s[q];
         const int a = x + 1, b = y + 1, c = z + 1;
         const double nz = (double)((msk[p] >> q) & 1);
-        const double lap = (sv3[c][b][a - 1] - 2 * sv3[c][b][a] + sv3[c][b][a + 1]) / (R.dx * R.dx) +
-                           (sv3[c][b - 1][a] - 2 * sv3[c][b][a] + sv3[c][b + 1][a]) / (R.dy * R.dy) +
-                           (sv3[c - 1][b][a] - 2 * sv3[c][b][a] + sv3[c + 1][b][a]) / (R.dz * R.dz);
+        const double s2 = 2 * sv3[c][b][a];
+        const double lap = div_by(sv3[c][b][a - 1] - s2 + sv3[c][b][a + 1], R.rx) +
+                           div_by(sv3[c][b - 1][a] - s2 + sv3[c][b + 1][a], R.ry) +
+                           div_by(sv3[c - 1][b][a] - s2 + sv3[c + 1][b][a], R.rz);
         const double dnoise = R.eta * D * nz * lap;
         sv3[c][b][a] += dnoise;
       }
@@ -455,11 +458,12 @@ __global__ void __launch_bounds__(64) k_noise_remove2(Geo g, double* __restrict_
     if (mine && x >= 0 && y < ye && x < xe) {
       const int a = x + 1, b = y + 1;
       const double nz = (double)((msk[x + T2 * y] >> q) & 1);
-      const double lgrad = (s[q][b][a] - s[q][b][a - 1]) / dx;
-      const double rgrad = (s[q][b][a + 1] - s[q][b][a]) / dx;
-      const double bgrad = (s[q][b][a] - s[q][b - 1][a]) / dy;
-      const double tgrad = (s[q][b + 1][a] - s[q][b][a]) / dy;
-      const double dv = R.eta * D * nz * ((rgrad - lgrad) / dx + (tgrad - bgrad) / dy);
+      const double lgrad = div_by(s[q][b][a] - s[q][b][a - 1], R.rx);
+      const double rgrad = div_by(s[q][b][a + 1] - s[q][b][a], R.rx);
+      const double bgrad = div_by(s[q][b][a] - s[q][b - 1][a], R.ry);
+      const double tgrad = div_by(s[q][b + 1][a] - s[q][b][a], R.ry);
+      const double dv =
+          R.eta * D * nz * (div_by(rgrad - lgrad, R.rx) + div_by(tgrad - bgrad, R.ry));
       s[q][b][a] += dv;
     }
     __syncwarp();  // each variable's steps stay within its own warp
@@ -566,8 +570,17 @@ int fst_noise_launch(const Geo& g, const fst_config& cf, double* U, int* noise,
       FST_LAUNCH(prof, "noise_detect", st, n,
                  k_noise_detect<2><<<nblk(centres, 256), 256, 0, st>>>(g, U, noise, A, ceq ? key : nullptr));
   }
-  RemoveArgs R{A.nvars, {A.vars[0], A.vars[1], A.vars[2]}, np.eta, dx, dy, dz,
-               skip_bound(np.eta, dx, dy, g.ndim == 3 ? dz : dy)};
+  RemoveArgs R{};
+  R.nvars = A.nvars;
+  for (int q = 0; q < 3; ++q) R.vars[q] = A.vars[q];
+  R.eta = np.eta;
+  R.dx = dx;
+  R.dy = dy;
+  R.dz = dz;
+  R.rx = fst64::recip_of(g.ndim == 3 ? dx * dx : dx);
+  R.ry = fst64::recip_of(g.ndim == 3 ? dy * dy : dy);
+  R.rz = fst64::recip_of(dz * dz);
+  R.safe = skip_bound(np.eta, dx, dy, g.ndim == 3 ? dz : dy);
   int* tiles = noise + g.sv;  // candidate tiles (fst_noise_ints)
   // the tile marks, then nt sweeps of one launch per tile diagonal
   auto sweeps = [&](cudaStream_t s, Prof* pr) {

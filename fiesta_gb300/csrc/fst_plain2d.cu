@@ -17,9 +17,11 @@
 // four C-equation variables with the fifth left unchanged, and no delta term
 // in the C-equation face tensor (src/ceq.hpp:200-245).  Built with
 // --fmad=false.
-#include "fst_internal.h"
+#include "fst_flux_dev.cuh"
 
 namespace {
+using fst64::div_by;
+using fst64::div_rn;
 
 // calculateRhoPT2D (src/secondary.hpp:60-107), computeVelocity2D
 // (src/velocity.hpp:85-99); maxWaveSpeed2D and maxCvar2D(var, 1)
@@ -36,9 +38,10 @@ __global__ void __launch_bounds__(256) k_prim2d(Geo g, Phys P, const double* __r
   if (c < sv) {
     double r = 0.0;
     for (int s = 0; s < P.ns; ++s) r = r + U[c + sv * (3 + s)];
+    const fst64::Recip rr = fst64::recip_of(r);
     double Cp = 0, Cv = 0, Cp2 = 0, Cv2 = 0;
     for (int s = 0; s < P.ns; ++s) {
-      double ys = U[c + sv * (3 + s)] / r;
+      double ys = div_by(U[c + sv * (3 + s)], rr);
       Cp = Cp + ys * P.cp_s[s];
       Cv = Cv + ys * P.cv_s[s];
       if (red) {
@@ -46,29 +49,29 @@ __global__ void __launch_bounds__(256) k_prim2d(Geo g, Phys P, const double* __r
         Cv2 = Cv2 + ys * P.cv2_s[s];
       }
     }
-    const double gam = Cp / Cv;
+    const double gam = div_rn(Cp, Cv);
     const double m0 = U[c], m1 = U[c + sv], E = U[c + 2 * sv];
-    const double p = (gam - 1) * (E - (0.5 / r) * (m0 * m0 + m1 * m1));
-    const double u = m0 / r, v = m1 / r;
+    const double p = (gam - 1) * (E - div_by(0.5, rr) * (m0 * m0 + m1 * m1));
+    const double u = div_by(m0, rr), v = div_by(m1, rr);
     rho[c] = r;
     pr[c] = p;
     if (met) {
       // computeGenVelocity2D (src/velocity.hpp:49-66), metric (a,b) at
       // met[c + sv*(a + 2b)]
-      vel[c] = met[c] * m0 / r + met[c + 2 * sv] * m1 / r;
-      vel[c + sv] = met[c + sv] * m0 / r + met[c + 3 * sv] * m1 / r;
+      vel[c] = div_by(met[c] * m0, rr) + div_by(met[c + 2 * sv] * m1, rr);
+      vel[c + sv] = div_by(met[c + sv] * m0, rr) + div_by(met[c + 3 * sv] * m1, rr);
     } else {
       vel[c] = u;
       vel[c + sv] = v;
     }
-    if (T) T[c] = p / ((Cp - Cv) * r);
-    if (nrg) nrg[c] = E / r - 0.5 * r * (u * u + v * v);
+    if (T) T[c] = div_rn(p, (Cp - Cv) * r);
+    if (nrg) nrg[c] = div_by(E, rr) - 0.5 * r * (u * u + v * v);
     if (red) {
       int i = (int)(c % g.sy), j = (int)(c / g.sy);
       bool in = i >= g.ng && i < g.ngi - g.ng && j >= g.ng && j < g.ngj - g.ng;
       if (in) {
-        const double gam2 = Cp2 / Cv2;
-        double a = sqrt(gam2 * p / r);
+        const double gam2 = div_rn(Cp2, Cv2);
+        double a = sqrt(div_by(gam2 * p, rr));
         double s = a + sqrt(m0 * m0 + m1 * m1);
         if (s > lS) lS = s;
         double ch = fabs(U[c + sv * (P.nv + 1)]);
@@ -86,33 +89,9 @@ __global__ void __launch_bounds__(256) k_prim2d(Geo g, Phys P, const double* __r
   }
 }
 
-// computeFluxWeno2D::weno (src/flux.hpp:37-63), double constants
-__device__ __forceinline__ double weno2d(double f1, double f2, double f3, double f4, double f5) {
-  const double eps = 1e-6;
-  double b1, b2, b3, w1, w2, w3, p1, p2, p3, a1, a2;
-  a1 = f1 - 2.0 * f2 + f3;
-  a2 = f1 - 4.0 * f2 + 3.0 * f3;
-  b1 = (13.0 / 12.0) * a1 * a1 + (0.25) * a2 * a2;
-  a1 = f2 - 2.0 * f3 + f4;
-  a2 = f2 - f4;
-  b2 = (13.0 / 12.0) * a1 * a1 + (0.25) * a2 * a2;
-  a1 = f3 - 2.0 * f4 + f5;
-  a2 = 3.0 * f3 - 4.0 * f4 + f5;
-  b3 = (13.0 / 12.0) * a1 * a1 + (0.25) * a2 * a2;
-  a1 = eps + b1;
-  w1 = (0.1) / (a1 * a1);
-  a1 = eps + b2;
-  w2 = (0.6) / (a1 * a1);
-  a1 = eps + b3;
-  w3 = (0.3) / (a1 * a1);
-  p1 = (1.0 / 3.0) * f1 + (-7.0 / 6.0) * f2 + (11.0 / 6.0) * f3;
-  p2 = (-1.0 / 6.0) * f2 + (5.0 / 6.0) * f3 + (1.0 / 3.0) * f4;
-  p3 = (1.0 / 3.0) * f3 + (5.0 / 6.0) * f4 + (-1.0 / 6.0) * f5;
-  return (w1 * p1 + w2 * p2 + w3 * p3) / (w1 + w2 + w3);
-}
-
-// computeFluxWeno2D::operator() (src/flux.hpp:65-105) for all v < nv,
-// face box [ng-1, ngi-ng) x [ng-1, ngj-ng).  F[(dir*nv + v)*sv + cell].
+// The centred and QUICK schemes (computeFluxCentered2D / computeFluxQuick2D,
+// src/flux.hpp:108-221) for all v < nv, face box [ng-1, ngi-ng) x [ng-1,
+// ngj-ng).  F[(dir*nv + v)*sv + cell].  (WENO5: fst_flux_dev.cuh.)
 __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __restrict__ U,
                                                 const double* __restrict__ rho,
                                                 const double* __restrict__ pr,
@@ -131,16 +110,18 @@ __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __r
     for (int dir = 0; dir < 2; ++dir) {
       const long long s = dir == 0 ? 1 : g.sy;
       const double* m = U + sv * dir;
-      const double uf = (0.0 - m[c + 2 * s] / rho[c + 2 * s] + 7.0 * m[c + s] / rho[c + s] +
-                         7.0 * m[c] / rho[c] - m[c - s] / rho[c - s]) /
-                        12.0;
-      const double pf = (0.0 - pr[c + 2 * s] + 7.0 * pr[c + s] + 7.0 * pr[c] - pr[c - s]) / 12.0;
+      const double uf =
+          div_rn(0.0 - div_rn(m[c + 2 * s], rho[c + 2 * s]) + div_rn(7.0 * m[c + s], rho[c + s]) +
+                     div_rn(7.0 * m[c], rho[c]) - div_rn(m[c - s], rho[c - s]),
+                 12.0);
+      const double pf =
+          div_rn(0.0 - pr[c + 2 * s] + 7.0 * pr[c + s] + 7.0 * pr[c] - pr[c - s], 12.0);
       const DivC dd = dir == 0 ? P.ddx : P.ddy;
       double* Fd = F + (long long)dir * P.nv * sv;
 #pragma unroll 1
       for (int v = 0; v < P.nv; ++v) {
         const double* q = U + sv * v;
-        double x1 = (0.0 - q[c + 2 * s] + 7.0 * q[c + s] + 7.0 * q[c] - q[c - s]) / 12.0;
+        double x1 = div_rn(0.0 - q[c + 2 * s] + 7.0 * q[c + s] + 7.0 * q[c] - q[c - s], 12.0);
         if (v == 2) x1 = x1 + pf;
         Fd[sv * v + c] = dd(uf * x1);
       }
@@ -151,38 +132,24 @@ __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __r
   for (int dir = 0; dir < 2; ++dir) {
     const long long s = dir == 0 ? 1 : g.sy;
     const double* vd = vel + sv * dir;
-    const double uf = (-vd[c + 2 * s] + 7.0 * vd[c + s] + 7.0 * vd[c] - vd[c - s]) / 12.0;
+    const double uf =
+        div_rn(-vd[c + 2 * s] + 7.0 * vd[c + s] + 7.0 * vd[c] - vd[c - s], 12.0);
     const DivC dd = dir == 0 ? P.ddx : P.ddy;
     double* Fd = F + (long long)dir * P.nv * sv;
 #pragma unroll 1
     for (int v = 0; v < P.nv; ++v) {
       const double* q = U + sv * v;
-      double f1, f2, f3, f4, f5;
       const long long o = uf < 0.0 ? -s : s;  // stencil runs upwind
-      const long long c0 = uf < 0.0 ? c + 3 * s : c - 2 * s;
-      f1 = q[c0]; f2 = q[c0 + o]; f3 = q[c0 + 2 * o]; f4 = q[c0 + 3 * o]; f5 = q[c0 + 4 * o];
-      const double p1 = pr[c0], p2 = pr[c0 + o], p3 = pr[c0 + 2 * o], p4 = pr[c0 + 3 * o],
-                   p5 = pr[c0 + 4 * o];
-      if (P.scheme == FST_SCHEME_QUICK) {
-        // computeFluxQuick2D (src/flux.hpp:169-221): three upwind values
-        // f1 = q(c0+o), f2 = q(c0+2o), f3 = q(c0+3o) of the same stencil
-        if (v == 2) {
-          f2 = f2 + p2; f3 = f3 + p3; f4 = f4 + p4;
-        } else if (!(fst_finite(p2) && fst_finite(p3) && fst_finite(p4))) {
-          f2 = f2 + 0.0 * p2; f3 = f3 + 0.0 * p3; f4 = f4 + 0.0 * p4;
-        }
-        Fd[sv * v + c] = dd(uf * (0.75 * f3 + 0.375 * f4 - 0.125 * f2));
-        continue;
-      }
+      const long long c0 = uf < 0.0 ? c + 2 * s : c - s;
+      double f1 = q[c0], f2 = q[c0 + o], f3 = q[c0 + 2 * o];
+      const double p1 = pr[c0], p2 = pr[c0 + o], p3 = pr[c0 + 2 * o];
       if (v == 2) {
-        f1 = f1 + p1; f2 = f2 + p2; f3 = f3 + p3; f4 = f4 + p4; f5 = f5 + p5;
-      } else if (!(fst_finite(p1) && fst_finite(p2) && fst_finite(p3) && fst_finite(p4) &&
-                   fst_finite(p5))) {
+        f1 = f1 + p1; f2 = f2 + p2; f3 = f3 + p3;
+      } else if (!(fst_finite(p1) && fst_finite(p2) && fst_finite(p3))) {
         // var + 0*p of the reference: NaN where a pressure is not finite
         f1 = f1 + 0.0 * p1; f2 = f2 + 0.0 * p2; f3 = f3 + 0.0 * p3;
-        f4 = f4 + 0.0 * p4; f5 = f5 + 0.0 * p5;
       }
-      Fd[sv * v + c] = dd(uf * weno2d(f1, f2, f3, f4, f5));
+      Fd[sv * v + c] = dd(uf * (0.75 * f2 + 0.375 * f3 - 0.125 * f1));
     }
   }
 }
@@ -232,7 +199,7 @@ __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __
   if (P.ceq) {
     const int nv = P.nv;
     const double maxCh = fst_unkey(red[1]);
-    const double alpha = (P.dxmag2 / (maxCh + 1.0e-6)) * P.alpha;  // src/cart2d.cpp:227
+    const double alpha = div_rn(P.dxmag2, maxCh + 1.0e-6) * P.alpha;  // src/cart2d.cpp:227
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
       const long long sf = f == 0 ? sx : sy;
@@ -242,6 +209,7 @@ __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __
       ct[0] = (U[c + sv * (nv + 2)] + U[c + sf + sv * (nv + 2)]) / 2.0;
       ct[1] = (U[c + sv * (nv + 3)] + U[c + sf + sv * (nv + 3)]) / 2.0;
       const double ctmag = (ct[0] * ct[0] + ct[1] * ct[1]) + 1.0e-6;
+      const fst64::Recip rmag = fst64::recip_of(ctmag);
 #pragma unroll
       for (int w = 0; w < 2; ++w) {
         const double* vw = vel + sv * w;
@@ -255,7 +223,7 @@ __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __
         }
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
-          const double m = alpha * r * chat * (ct[f] * ct[d]) / ctmag;
+          const double m = div_by(alpha * r * chat * (ct[f] * ct[d]), rmag);
           MF[(long long)((f * 2 + d) * 2 + w) * sv + c] = m * gr[d];
         }
       }
@@ -300,20 +268,22 @@ __global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __r
     // applyGenPressureGradient2D (src/presgrad.hpp:148-190)
     auto d4m = [&](long long st, int a, int w) {
       const double* m = met + sv * (a + 2 * w);
-      return (pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
-              8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st]) /
-             12.0;
+      return div_rn(pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
+                        8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st],
+                    12.0);
     };
     R0 = R0 - (d4m(sx, 0, 0) + d4m(sy, 1, 0));
     R1 = R1 - (d4m(sx, 0, 1) + d4m(sy, 1, 1));
   } else {
-    const double dxp = (pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]) / P.d12x;
-    const double dyp = (pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]) / P.d12y;
+    const double dxp =
+        P.d12x(pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]);
+    const double dyp =
+        P.d12y(pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]);
     R0 -= dxp;
     R1 -= dyp;
   }
   if (P.buoyancy) {
-    const double vb = U[c + sv] / U[c + 3 * sv];
+    const double vb = div_rn(U[c + sv], U[c + 3 * sv]);
     const double rhop = rho[c] - P.rho_ref;
     const double eps = 1e-6;
     if (rhop >= eps || rhop <= -eps) {
@@ -343,8 +313,8 @@ __global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __r
     R2 = R2 + c1 - c2;
   }
   if (P.ceq) {
-    auto d4 = [&](const double* a, long long st, double d12) {
-      return (a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]) / d12;
+    auto d4 = [&](const double* a, long long st, const DivC& d12) {
+      return d12(a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]);
     };
     const double dxr = d4(rho, sx, P.d12x), dyr = d4(rho, sy, P.d12y);
     const double dxe = d4(nrg, sx, P.d12x), dye = d4(nrg, sy, P.d12y);
@@ -361,7 +331,7 @@ __global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __r
     G[2] = -dyr;
     G[3] = dxr;
     const double maxS = fst_unkey(red[0]);
-    const double src = maxS / (P.eps * P.dxmag);
+    const double src = div_rn(maxS, P.eps * P.dxmag);
     const double dif = P.kap * maxS * P.dxmag;
 #pragma unroll
     for (int n = 0; n < 4; ++n) {
@@ -431,7 +401,10 @@ int fst_plain2d_stage(const Geo& g, const Phys& P, const Plain2DBufs& b, const d
   const dim3 bf(32, 4, 1);
   const dim3 gf(cdiv(g.nci + 1, 32), cdiv(g.ncj + 1, 4), 1);
   FST_LAUNCH(prof, "flux2d", st, n,
-             k_flux2d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.F));
+             if (P.scheme == FST_SCHEME_WENO5)
+               fstflux::launch<false>(g, P, 2, Uin, b.pr, b.vel, b.F, st);
+             else
+               k_flux2d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.F));
   if (P.visc || P.ceq) {
     FST_LAUNCH(prof, "faces2d", st, n,
                k_faces2d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.T, b.red, b.S, b.Q, b.MF));

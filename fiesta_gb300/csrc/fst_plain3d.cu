@@ -25,9 +25,11 @@
 // performs on every value it stores, in the same order.  Built with
 // --fmad=false so no a*b+c is contracted: results match the reference's FP64
 // run bit for bit.
-#include "fst_internal.h"
+#include "fst_flux_dev.cuh"
 
 namespace {
+using fst64::div_by;
+using fst64::div_rn;
 
 // ---------------------------------------------------------------------------
 // k_prim3d: calculateRhoPT3D (src/secondary.hpp:109-151), computeVelocity3D
@@ -46,17 +48,18 @@ __global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __r
   if (c < sv) {
     double r = 0.0;
     for (int s = 0; s < P.ns; ++s) r = r + U[c + sv * (4 + s)];
+    const fst64::Recip rr = fst64::recip_of(r);
     double Cp = 0, Cv = 0;
     for (int s = 0; s < P.ns; ++s) {
-      double ys = U[c + sv * (4 + s)] / r;
+      double ys = div_by(U[c + sv * (4 + s)], rr);
       Cp = Cp + ys * P.cp_s[s];
       Cv = Cv + ys * P.cv_s[s];
       if (Y) Y[c + sv * s] = ys;
     }
-    const double gam = Cp / Cv;
+    const double gam = div_rn(Cp, Cv);
     const double m0 = U[c], m1 = U[c + sv], m2 = U[c + 2 * sv], E = U[c + 3 * sv];
-    const double p = (gam - 1) * (E - (0.5 / r) * (m0 * m0 + m1 * m1 + m2 * m2));
-    const double u = m0 / r, v = m1 / r, w = m2 / r;
+    const double p = (gam - 1) * (E - div_by(0.5, rr) * (m0 * m0 + m1 * m1 + m2 * m2));
+    const double u = div_by(m0, rr), v = div_by(m1, rr), w = div_by(m2, rr);
     rho[c] = r;
     pr[c] = p;
     if (met) {
@@ -65,23 +68,24 @@ __global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __r
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
         const double* M = met + c + sv * a;
-        vel[c + sv * a] = M[0] * m0 / r + M[3 * sv] * m1 / r + M[6 * sv] * m2 / r;
+        vel[c + sv * a] =
+            div_by(M[0] * m0, rr) + div_by(M[3 * sv] * m1, rr) + div_by(M[6 * sv] * m2, rr);
       }
     } else {
       vel[c] = u;
       vel[c + sv] = v;
       vel[c + 2 * sv] = w;
     }
-    if (T) T[c] = p / ((Cp - Cv) * r);
+    if (T) T[c] = div_rn(p, (Cp - Cv) * r);
     // specific internal energy of calculateRhoGrad::nrg (src/ceq3d.hpp:137-141)
-    if (nrg) nrg[c] = E / r - 0.5 * r * (u * u + v * v + w * w);
+    if (nrg) nrg[c] = div_by(E, rr) - 0.5 * r * (u * u + v * v + w * w);
     if (red) {
       int i = (int)(c % g.sy), j = (int)((c / g.sy) % g.ngj), k = (int)(c / g.sz);
       bool in = i >= g.ng && i < g.ngi - g.ng && j >= g.ng && j < g.ngj - g.ng &&
                 k >= g.ng && k < g.ngk - g.ng;
       if (in) {
-        double a = sqrt(gam * p / r);
-        double s = a + sqrt(m0 * m0 + m1 * m1 + m2 * m2) / r;
+        double a = sqrt(div_by(gam * p, rr));
+        double s = a + div_by(sqrt(m0 * m0 + m1 * m1 + m2 * m2), rr);
         if (s > lS) lS = s;
         double ch = fabs(U[c + sv * (P.nv + 1)]);
         if (ch > lC) lC = ch;
@@ -94,79 +98,6 @@ __global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __r
     if ((threadIdx.x & 31) == 0) {
       atomicMax(&red[0], fst_key(lS));
       atomicMax(&red[1], fst_key(lC));
-    }
-  }
-}
-
-// calculateFluxesG::weno (src/flux.hpp:241-266), constants as float literals
-__device__ __forceinline__ double weno3d(double f1, double f2, double f3, double f4, double f5) {
-  const double eps = 0.000001;
-  double b1, b2, b3, w1, w2, w3, p1, p2, p3, a1, a2;
-  a1 = f1 - 2.0f * f2 + f3;
-  a2 = f1 - 4.0f * f2 + 3.0f * f3;
-  b1 = (13.0f / 12.0f) * a1 * a1 + (0.25f) * a2 * a2;
-  a1 = f2 - 2.0 * f3 + f4;
-  a2 = f2 - f4;
-  b2 = (13.0f / 12.0f) * a1 * a1 + (0.25f) * a2 * a2;
-  a1 = f3 - 2.0 * f4 + f5;
-  a2 = 3.0 * f3 - 4.0 * f4 + f5;
-  b3 = (13.0f / 12.0f) * a1 * a1 + (0.25f) * a2 * a2;
-  a1 = eps + b1;
-  w1 = (0.1f) / (a1 * a1);
-  a1 = eps + b2;
-  w2 = (0.6f) / (a1 * a1);
-  a1 = eps + b3;
-  w3 = (0.3f) / (a1 * a1);
-  p1 = (1.0f / 3.0f) * f1 + (-7.0f / 6.0f) * f2 + (11.0f / 6.0f) * f3;
-  p2 = (-1.0f / 6.0f) * f2 + (5.0f / 6.0f) * f3 + (1.0f / 3.0f) * f4;
-  p3 = (1.0f / 3.0f) * f3 + (5.0f / 6.0f) * f4 + (-1.0f / 6.0f) * f5;
-  return (w1 * p1 + w2 * p2 + w3 * p3) / (w1 + w2 + w3);
-}
-
-// ---------------------------------------------------------------------------
-// k_flux3d: calculateFluxesG::operator() (src/flux.hpp:268-309) for all v<nv
-// on the x, y and z faces at (i+1/2, j, k), (i, j+1/2, k), (i, j, k+1/2),
-// face index box [ng-1, ngi-ng) in every dimension.
-// F layout: F[(dir*nv + v)*sv + cell].
-// The stencil value is var + (v==3)*p.  For v != 3 that is var + 0*p: var
-// itself when the six pressures are finite (signed zeros aside, which never
-// change a nonzero result), and NaN otherwise; the add is only executed in
-// the second case, so NaN propagates exactly as in the reference.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_flux3d(Geo g, Phys P, const double* __restrict__ U,
-                                                const double* __restrict__ pr,
-                                                const double* __restrict__ vel,
-                                                double* __restrict__ F) {
-  const int i = g.ng - 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = g.ng - 1 + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = g.ng - 1 + blockIdx.z;
-  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || k >= g.ngk - g.ng) return;
-  const long long c = fst_idx(g, i, j, k);
-  const long long sv = g.sv;
-#pragma unroll 1
-  for (int dir = 0; dir < 3; ++dir) {
-    const long long s = dir == 0 ? 1 : dir == 1 ? g.sy : g.sz;
-    const double* vd = vel + sv * dir;
-    const double uf = (-vd[c + 2 * s] + 7.0f * vd[c + s] + 7.0f * vd[c] - vd[c - s]) / 12.0f;
-    const DivC dd = dir == 0 ? P.ddx : dir == 1 ? P.ddy : P.ddz;
-    double* Fd = F + (long long)dir * P.nv * sv;
-    const double p1 = pr[c + 3 * s], p2 = pr[c + 2 * s], p3 = pr[c + s], p4 = pr[c],
-                 p5 = pr[c - s], p6 = pr[c - 2 * s];
-    const bool pfin = fst_finite(p1) && fst_finite(p2) && fst_finite(p3) && fst_finite(p4) &&
-                      fst_finite(p5) && fst_finite(p6);
-#pragma unroll 1
-    for (int v = 0; v < P.nv; ++v) {
-      const double* q = U + sv * v;
-      double f1 = q[c + 3 * s], f2 = q[c + 2 * s], f3 = q[c + s], f4 = q[c], f5 = q[c - s],
-             f6 = q[c - 2 * s];
-      if (v == 3) {
-        f1 = f1 + p1; f2 = f2 + p2; f3 = f3 + p3; f4 = f4 + p4; f5 = f5 + p5; f6 = f6 + p6;
-      } else if (!pfin) {
-        f1 = f1 + 0.0 * p1; f2 = f2 + 0.0 * p2; f3 = f3 + 0.0 * p3;
-        f4 = f4 + 0.0 * p4; f5 = f5 + 0.0 * p5; f6 = f6 + 0.0 * p6;
-      }
-      double wv = uf < 0.0 ? weno3d(f1, f2, f3, f4, f5) : weno3d(f6, f5, f4, f3, f2);
-      Fd[sv * v + c] = dd(uf * wv);
     }
   }
 }
@@ -197,7 +128,7 @@ __global__ void __launch_bounds__(128) k_faces3d(Geo g, Phys P, const double* __
   double alpha = 0.0;
   if (P.ceq) {
     const double maxCh = fst_unkey(red[1]);
-    alpha = (P.dxmag2 / (maxCh + 1.0e-6)) * P.alpha;  // src/cart3d.cpp:285
+    alpha = div_rn(P.dxmag2, maxCh + 1.0e-6) * P.alpha;  // src/cart3d.cpp:285
   }
 #pragma unroll
   for (int f = 0; f < 3; ++f) {
@@ -244,10 +175,11 @@ __global__ void __launch_bounds__(128) k_faces3d(Geo g, Phys P, const double* __
       cmag += cn[0] * cn[0];
       cmag += cn[1] * cn[1];
       cmag += cn[2] * cn[2];
+const fst64::Recip rmag = fst64::recip_of(cmag);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
         const double dirac = f == d ? 1.0 : 0.0;
-        const double M = dirac - (cn[f] * cn[d]) / cmag;
+        const double M = dirac - div_by(cn[f] * cn[d], rmag);
         const double base = alpha * r * chat * M;
         double* MFd = MF + (long long)((f * 3 + d) * 3) * sv + c;
 #pragma unroll
@@ -306,23 +238,26 @@ __global__ void __launch_bounds__(128) k_cell3d(Geo g, Phys P, const double* __r
     // differences of p * m(a, w) along each computational direction a
     auto d4m = [&](long long st, int a, int w) {
       const double* m = met + sv * (a + 3 * w);
-      return (pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
-              8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st]) /
-             12.0;
+      return div_rn(pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
+                        8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st],
+                    12.0);
     };
     R0 = R0 - (d4m(sx, 0, 0) + d4m(sy, 1, 0) + d4m(sz, 2, 0));
     R1 = R1 - (d4m(sx, 0, 1) + d4m(sy, 1, 1) + d4m(sz, 2, 1));
     R2 = R2 - (d4m(sx, 0, 2) + d4m(sy, 1, 2) + d4m(sz, 2, 2));
   } else {  // pressure gradient; the reference uses dz = cd(2) for the z term
-    const double dxp = (pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]) / P.d12x;
-    const double dyp = (pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]) / P.d12y;
-    const double dzp = (pr[c - 2 * sz] - 8.0 * pr[c - sz] + 8.0 * pr[c + sz] - pr[c + 2 * sz]) / P.d12pz;
+    const double dxp =
+        P.d12x(pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]);
+    const double dyp =
+        P.d12y(pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]);
+    const double dzp =
+        P.d12pz(pr[c - 2 * sz] - 8.0 * pr[c - sz] + 8.0 * pr[c + sz] - pr[c + 2 * sz]);
     R0 = R0 - dxp;
     R1 = R1 - dyp;
     R2 = R2 - dzp;
   }
   if (P.buoyancy) {
-    const double vb = U[c + sv] / rho[c];
+    const double vb = div_rn(U[c + sv], rho[c]);
     const double rhop = rho[c] - P.rho_ref;
     const double f = -P.g * rhop;
     R1 += f;
@@ -357,8 +292,8 @@ __global__ void __launch_bounds__(128) k_cell3d(Geo g, Phys P, const double* __r
   }
   if (P.ceq) {
     // calculateRhoGrad
-    auto d4 = [&](const double* a, long long st, double d12) {
-      return (a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]) / d12;
+    auto d4 = [&](const double* a, long long st, const DivC& d12) {
+      return d12(a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]);
     };
     const double dxr = d4(rho, sx, P.d12x), dyr = d4(rho, sy, P.d12y), dzr = d4(rho, sz, P.d12z);
     const double dxe = d4(nrg, sx, P.d12x), dye = d4(nrg, sy, P.d12y), dze = d4(nrg, sz, P.d12z);
@@ -377,7 +312,7 @@ __global__ void __launch_bounds__(128) k_cell3d(Geo g, Phys P, const double* __r
     G[4] = dzr;
     // updateCeq
     const double maxS = fst_unkey(red[0]);
-    const double src = maxS / (P.eps * P.dxmag);
+    const double src = div_rn(maxS, P.eps * P.dxmag);
     const double dif = P.kap * maxS * P.dxmag;
 #pragma unroll
     for (int n = 0; n < 5; ++n) {
@@ -452,7 +387,7 @@ int fst_plain3d_stage(const Geo& g, const Phys& P, const Plain3DBufs& b, const d
                                                        P.ceq ? b.red : nullptr, b.met));
   const dim3 bf(32, 4, 1);
   const dim3 gf(cdiv(g.nci + 1, 32), cdiv(g.ncj + 1, 4), g.nck + 1);
-  FST_LAUNCH(prof, "flux3d", st, n, k_flux3d<<<gf, bf, 0, st>>>(g, P, Uin, b.pr, b.vel, b.F));
+  FST_LAUNCH(prof, "flux3d", st, n, fstflux::launch<true>(g, P, 3, Uin, b.pr, b.vel, b.F, st));
   if (P.visc || P.ceq) {
     FST_LAUNCH(prof, "faces3d", st, n,
                k_faces3d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.Y, b.red, b.S, b.MF));
