@@ -20,7 +20,7 @@
 // registers and its global loads few; the cost is reading the velocities
 // three times and the momenta/energy of U_new twice.
 //
-// Face kernels: blocks of 32x8 threads march along k (16 planes).  Thread
+// Face kernels: blocks of 32x8 threads march along k (up to 16 planes).  Thread
 // (tx, ty) owns column (i0-1+tx, j0-1+ty); it computes the face at i+1/2
 // from the x-stencil, the face at j+1/2 from the y-stencil and, for the
 // 31x7 interior columns, the face at k+1/2; the left x face comes from
@@ -67,7 +67,7 @@ using namespace fstm;
 using namespace fsttma;
 
 constexpr int HX = 40, HY = 13, PL = HX * HY;  // one field of a plane tile (floats)
-constexpr int KZ3 = 16;                        // planes per block along k
+constexpr int KZ3 = 16;                        // planes per block along k, at most
 constexpr int NBUF = 3;                        // plane tiles in flight per block
 constexpr int NRING = 5;                       // velocity planes k-2 .. k+2
 
@@ -218,7 +218,7 @@ __device__ __forceinline__ float d4pairz(const float h[5], const float l[5], flo
 __global__ void __launch_bounds__(TX * TY, 3)
     k_mcell3d(const __grid_constant__ Mixed3DMaps maps, Geo g, Geo gq, Phys P, MixedView M,
               const double* Uold, double* Unew, double coef, double* __restrict__ Rout,
-              unsigned int* __restrict__ err) {
+              unsigned int* __restrict__ err, int kz) {
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = aligned_smem(smdyn);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(TX * TY, 3)
   const int tid = threadIdx.y * TX + threadIdx.x;
   const Place pl = place_cells(g);
   const int i = pl.i, j = pl.j;
-  const int kc0 = g.ng + (int)blockIdx.z * KZ3;
-  const int kc1 = min(kc0 + KZ3, g.ngk - g.ng);
+  const int kc0 = g.ng + (int)blockIdx.z * kz;
+  const int kc1 = min(kc0 + kz, g.ngk - g.ng);
   const bool cell = i < g.ngi - g.ng && j < g.ngj - g.ng;
   const long long cq0 = (long long)i + gq.sy * j;
   const long long c0 = (long long)i + g.sy * j;
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
     k_mceq3d(const __grid_constant__ Mixed3DMaps maps, Geo g, Geo gq, Phys P, MixedView M,
              const unsigned long long* __restrict__ red, const double* Uold, double* Unew,
              double coef, double* __restrict__ Rout, unsigned int* __restrict__ err,
-             float* __restrict__ Cn, unsigned long long* __restrict__ red_n) {
+             float* __restrict__ Cn, unsigned long long* __restrict__ red_n, int kz) {
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = aligned_smem(smdyn);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
@@ -351,8 +351,8 @@ __global__ void __launch_bounds__(TX * TY, 2)
   const int tid = threadIdx.y * TX + threadIdx.x;
   const Place pl = place_cells(g);
   const int i = pl.i, j = pl.j;
-  const int kc0 = g.ng + (int)blockIdx.z * KZ3;
-  const int kc1 = min(kc0 + KZ3, g.ngk - g.ng);
+  const int kc0 = g.ng + (int)blockIdx.z * kz;
+  const int kc1 = min(kc0 + kz, g.ngk - g.ng);
   const bool cell = i < g.ngi - g.ng && j < g.ngj - g.ng;
   const long long cq0 = (long long)i + gq.sy * j;
   const long long c0 = (long long)i + g.sy * j;
@@ -540,7 +540,7 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
               const unsigned char* __restrict__ smap, const double* Uold, double* Unew,
               double coef, double* __restrict__ Rout, int sb, int nsk,
               unsigned int* __restrict__ err, Prim3Out On,
-              unsigned long long* __restrict__ red_n) {
+              unsigned long long* __restrict__ red_n, int kz) {
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = aligned_smem(smdyn);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
@@ -550,8 +550,8 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const Place pl = place_faces(g);
   const int i = pl.i, j = pl.j;
-  const int kc0 = g.ng + (int)blockIdx.z * KZ3;
-  const int kc1 = min(kc0 + KZ3, g.ngk - g.ng);
+  const int kc0 = g.ng + (int)blockIdx.z * kz;
+  const int kc1 = min(kc0 + kz, g.ngk - g.ng);
   const bool fi = i <= g.ngi - g.ng - 1;
   const bool fj = j <= g.ngj - g.ng - 1;
   const bool ci = tx >= 1 && i >= g.ng && i < g.ngi - g.ng;
@@ -793,7 +793,7 @@ __global__ void __launch_bounds__(TX * TY, 2)
     k_mmom3d(const __grid_constant__ Mixed3DMaps maps, Geo g, Geo gq, Phys P, MixedView M,
              const unsigned long long* __restrict__ red, const unsigned char* __restrict__ smap,
              double* Unew, double coef, double* __restrict__ Rout,
-             unsigned int* __restrict__ err) {
+             unsigned int* __restrict__ err, int kz) {
   extern __shared__ __align__(128) unsigned char smdyn[];
   unsigned char* smraw = aligned_smem(smdyn);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);  // [0..2] tiles, [3..7] velocity ring
@@ -805,8 +805,8 @@ __global__ void __launch_bounds__(TX * TY, 2)
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
   const Place pl = place_faces(g);
   const int i = pl.i, j = pl.j;
-  const int kc0 = g.ng + (int)blockIdx.z * KZ3;
-  const int kc1 = min(kc0 + KZ3, g.ngk - g.ng);
+  const int kc0 = g.ng + (int)blockIdx.z * kz;
+  const int kc1 = min(kc0 + kz, g.ngk - g.ng);
   const bool fi = i <= g.ngi - g.ng - 1;
   const bool fj = j <= g.ngj - g.ng - 1;
   const bool ci = tx >= 1 && i >= g.ng && i < g.ngi - g.ng;
@@ -1039,6 +1039,28 @@ __global__ void __launch_bounds__(TX * TY, 2)
 
 inline unsigned cdiv3(long long a, int b) { return (unsigned)((a + b - 1) / b); }
 
+// Planes per block along k for `tiles` (x, y) tiles.  A block costs about three
+// planes of start-up (window loads, first TMA planes, first z face) besides its
+// own, and two blocks fit an SM; the fewest planes x waves wins, the longer march
+// on a tie.  Large grids take KZ3.  Measured per step against KZ3 everywhere:
+// 33x20x18 235 -> 88 us, 61x50x37 244 -> 118, 96x80x64 465 -> 367, 128^3 1229 ->
+// 1206, 160^3 2189 -> 2088, 256^3 the same (fewer planes lose there: 8 planes
+// 2.5 %, 4 planes 9 %).
+int plan_kz(long long tiles, int nck) {
+  const long long slots = 2 * 152;
+  int best = KZ3;
+  long long cost = -1;
+  for (int kz = KZ3; kz >= 1; --kz) {
+    const long long blocks = tiles * ((nck + kz - 1) / kz);
+    const long long c = (blocks + slots - 1) / slots * (3 + kz);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = kz;
+    }
+  }
+  return best;
+}
+
 size_t spec_smem(int nsc) {
   return ALIGN_SLACK + BAR_BYTES +
          sizeof(float) * (NBUF * (size_t)spec_layout(nsc).size + 2 * (size_t)TY * TX * nsc);
@@ -1059,7 +1081,9 @@ template <int NS, bool HYB>
 int launch_spec(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                 const unsigned char* smooth, const double* Uold, double* Unew, double coef,
                 double* Rout, cudaStream_t st, bool fused) {
-  const dim3 grd(cdiv3(g.nci, TX - 1), cdiv3(g.ncj, TY - 1), cdiv3(g.nck, KZ3));
+  const unsigned nx = cdiv3(g.nci, TX - 1), ny = cdiv3(g.ncj, TY - 1);
+  const int kz = plan_kz((long long)nx * ny, g.nck);
+  const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = spec_smem(NS);
   if (fused) {  // one launch over all species, with the equation-of-state epilogue
     const PrimSet& A = b.alt;
@@ -1068,7 +1092,7 @@ int launch_spec(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView
     cudaFuncSetAttribute(k_mspec3d<NS, HYB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sm);
     k_mspec3d<NS, HYB, true><<<grd, dim3(TX, TY), sm, st>>>(
-        *b.maps3d, g, b.gq, P, M, smooth, Uold, Unew, coef, Rout, 0, g.ns, b.dev_err, On, A.red);
+        *b.maps3d, g, b.gq, P, M, smooth, Uold, Unew, coef, Rout, 0, g.ns, b.dev_err, On, A.red, kz);
     return 1;
   }
   cudaFuncSetAttribute(k_mspec3d<NS, HYB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1078,7 +1102,7 @@ int launch_spec(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView
     const int nsk = g.ns - sb < NS ? g.ns - sb : NS;
     k_mspec3d<NS, HYB, false><<<grd, dim3(TX, TY), sm, st>>>(*b.maps3d, g, b.gq, P, M, smooth,
                                                              Uold, Unew, coef, Rout, sb, nsk,
-                                                             b.dev_err, Prim3Out{}, nullptr);
+                                                             b.dev_err, Prim3Out{}, nullptr, kz);
     ++n;
   }
   return n;
@@ -1101,31 +1125,37 @@ template <bool HYB>
 void launch_mom(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                 const unsigned char* smooth, double* Unew, double coef, double* Rout,
                 cudaStream_t st) {
-  const dim3 grd(cdiv3(g.nci, TX - 1), cdiv3(g.ncj, TY - 1), cdiv3(g.nck, KZ3));
+  const unsigned nx = cdiv3(g.nci, TX - 1), ny = cdiv3(g.ncj, TY - 1);
+  const int kz = plan_kz((long long)nx * ny, g.nck);
+  const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = mom_smem(P.visc != 0, P.ceq != 0);
   cudaFuncSetAttribute(k_mmom3d<HYB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_mmom3d<HYB><<<grd, dim3(TX, TY), sm, st>>>(*b.maps3d, g, b.gq, P, M, b.red, smooth, Unew,
-                                              coef, Rout, b.dev_err);
+                                              coef, Rout, b.dev_err, kz);
 }
 
 void launch_cell(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                  const double* Uold, double* Unew, double coef, double* Rout, cudaStream_t st) {
-  const dim3 grd(cdiv3(g.nci, TX), cdiv3(g.ncj, TY), cdiv3(g.nck, KZ3));
+  const unsigned nx = cdiv3(g.nci, TX), ny = cdiv3(g.ncj, TY);
+  const int kz = plan_kz((long long)nx * ny, g.nck);
+  const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = cell_smem();
   cudaFuncSetAttribute(k_mcell3d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_mcell3d<<<grd, dim3(TX, TY), sm, st>>>(*b.maps3d, g, b.gq, P, M, Uold, Unew, coef, Rout,
-                                          b.dev_err);
+                                          b.dev_err, kz);
 }
 
 void launch_ceq(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                 const double* Uold, double* Unew, double coef, double* Rout, cudaStream_t st,
                 bool fused) {
-  const dim3 grd(cdiv3(g.nci, TX), cdiv3(g.ncj, TY), cdiv3(g.nck, KZ3));
+  const unsigned nx = cdiv3(g.nci, TX), ny = cdiv3(g.ncj, TY);
+  const int kz = plan_kz((long long)nx * ny, g.nck);
+  const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = ceq_smem();
   cudaFuncSetAttribute(k_mceq3d, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   k_mceq3d<<<grd, dim3(TX, TY), sm, st>>>(*b.maps3d, g, b.gq, P, M, b.red, Uold, Unew, coef,
                                          Rout, b.dev_err, fused ? b.alt.C : nullptr,
-                                         fused ? b.alt.red : nullptr);
+                                         fused ? b.alt.red : nullptr, kz);
 }
 
 // species per k_mspec3d launch: all of them up to 5, else chunks of 4
