@@ -203,6 +203,9 @@ def algorithmic_bytes(kernel, cfg):
     tab["mspec3d_eos"] = tab["mspec3d"] + inner * (8 * 4 + prim_out)
     tab["mprim3d_shell"] = (allc - inner) * (8 * nvt + 4 * (nv + 1 + 3 + 2 + visc
                                                             + (11 if ceq else 0)) + 8 * buoy)
+    # the shell pass with the boundary fill: also writes the state's ghost cells in
+    # one of the two stages
+    tab["mfill3d_shell"] = tab["mprim3d_shell"] + (allc - inner) * 4 * nvt
     # generalized grids (plain FP64): primitives read the 9 metrics and write
     # rho, p and the contravariant velocity; the cell pass reads the fluxes,
     # p and the 9 metrics once each

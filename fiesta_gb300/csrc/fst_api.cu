@@ -475,6 +475,7 @@ int fst_create(const fst_config* cfg, fst_ctx** out) {
     rc = fst_mixed_alloc(*cfg, g, c->bm, [&](void** p, size_t bytes) { return alloc(c, p, bytes); },
                          &why);
     if (rc && !why.empty()) fail(c, rc, why);
+    c->bm.rule = fstbc::ghost_rule(g, *cfg);
   }
   // zero state like a fresh Kokkos View; zero work arrays so that entries
   // outside each kernel's range read as the reference's zero-initialised ones
@@ -665,19 +666,35 @@ namespace {
 // c->bm.dl applies to stage 2 only.
 int one_step(fst_ctx* c) {
   int rc = FST_OK;
-  const bool two_d = c->g.ndim == 2;
+  const Geo& g = c->g;
+  const bool cart3 = g.ndim == 3 && !c->gen;
+  // Boundary conditions before a stage on U (3D), or left to the stage's shell
+  // pass: fused mixed stages whose ghost cells are copies of interior ones.  The
+  // stage-1 buffer's ghosts then exist as primitives only.
+  auto ghosts = [&](double* U) {
+    c->bm.fill = c->bm.fused && c->bm.fused_for == U && c->bm.rule.direct &&
+                 fst_shell_count(g) < (1LL << 31);
+    c->bm.fill_state = U == c->Ua;
+    return c->bm.fill ? FST_OK : bcs(c, U);
+  };
+  // Stage 1 copies the ghosts into its buffer (U + (0.5 dt) 0, src/rk.cpp:42-50)
+  // where they are read: always in 2D and on generalized grids, in 3D only where
+  // a fill with fewer cells than ghost layers reads ghosts.
+  const bool keep = !cart3 || g.nci < g.ng || g.ncj < g.ng || g.nck < g.ng;
   // gen2d / gen3d apply no boundary conditions (src/gen2d.cpp:132-134,
   // src/gen3d.cpp:109, 338-370)
-  if (two_d && !c->gen) rc = bcs(c, c->Ua);  // cart2d_func::preStep
-  if (!rc && !two_d && !c->gen) rc = bcs(c, c->Ua);
+  if (g.ndim == 2 && !c->gen) rc = bcs(c, c->Ua);  // cart2d_func::preStep
+  if (cart3) rc = ghosts(c->Ua);
   c->bm.stage = 1;
   MixedDownload* dl = c->bm.dl;
   c->bm.dl = nullptr;
-  if (!rc) rc = stage(c, c->Ua, c->Ua, c->Ub, c->P.hdt, nullptr, true);
+  if (!rc) rc = stage(c, c->Ua, c->Ua, c->Ub, c->P.hdt, nullptr, keep);
   c->bm.dl = dl;
-  if (!rc && !two_d && !c->gen) rc = bcs(c, c->Ub);
+  c->bm.fill = false;
+  if (!rc && cart3) rc = ghosts(c->Ub);
   c->bm.stage = 2;
   if (!rc) rc = stage(c, c->Ub, c->Ua, c->Ua, c->P.dt, nullptr, false);
+  c->bm.fill = false;
   if (rc) return rc;
   c->bm.step += 1;
   c->stats.steps += 1;

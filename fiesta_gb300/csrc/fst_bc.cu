@@ -9,7 +9,9 @@
 // are separate launches because later axes read ghosts written by earlier
 // ones; the two faces of an axis share a launch when they touch disjoint
 // cells.  One thread owns one ghost line and runs the reference's per-line
-// loop in the reference's order.
+// loop in the reference's order.  Where the sequence amounts to one copy per ghost
+// cell (no hydrostatic face, at least ng cells per axis) a single launch makes
+// those copies instead, with the same values.
 //
 // Built with --fmad=false: the hydrostatic energy extrapolation must round
 // exactly as the reference does.
@@ -42,6 +44,28 @@ __global__ void k_face(Geo g, double* __restrict__ U, int axis, int side, int ty
   fstbc::face_line(g, U, axis, sd, sd ? type_hi : type, (int)(t % na), (int)(t / na));
 }
 
+// Every ghost cell in one launch (fstbc::GhostRule): a thread copies VC variables
+// of one ghost cell, its loads in flight together.
+constexpr int VC = 5;
+__global__ void __launch_bounds__(128) k_ghosts(Geo g, fstbc::GhostRule r, double* __restrict__ U,
+                                                int nshell) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= nshell) return;
+  int i, j, k;
+  fst_shell_cell(g, t, i, j, k);
+  const long long dst = fst_idx(g, i, j, k);
+  const unsigned flip = fstbc::ghost_source(g, r, i, j, k);
+  const long long src = fst_idx(g, i, j, k);
+  const int v0 = blockIdx.y * VC;
+  double x[VC];
+#pragma unroll
+  for (int q = 0; q < VC; ++q)
+    if (v0 + q < g.nvt) x[q] = U[src + g.sv * (v0 + q)];
+#pragma unroll
+  for (int q = 0; q < VC; ++q)
+    if (v0 + q < g.nvt) U[dst + g.sv * (v0 + q)] = fstbc::ghost_value(x[q], flip, v0 + q);
+}
+
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // Reset n reduction words to v on the stream (in place of a copy from host
@@ -62,6 +86,14 @@ void fst_fill_keys(unsigned long long* p, int n, unsigned long long v, cudaStrea
 int fst_launch_bcs(const Geo& g, const fst_config& cf, double* U, cudaStream_t stream, Prof* prof) {
   int launches = 0;
   const int B = 128;
+  const fstbc::GhostRule rule = fstbc::ghost_rule(g, cf);
+  const long long shell = fst_shell_count(g);
+  if (rule.direct && shell < (1LL << 31)) {
+    FST_LAUNCH(prof, "bc_ghosts", stream, launches,
+               k_ghosts<<<dim3(nblk(shell, B), nblk(g.nvt, VC)), B, 0, stream>>>(g, rule, U,
+                                                                                 (int)shell));
+    return launches;
+  }
   const bool per[3] = {cf.xper != 0, cf.yper != 0, g.ndim == 3 && cf.zper != 0};
   for (int ax = 0; ax < g.ndim; ++ax) {
     if (!per[ax]) continue;

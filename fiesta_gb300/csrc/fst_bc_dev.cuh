@@ -102,4 +102,61 @@ __device__ __forceinline__ void face_line(const Geo& g, double* __restrict__ U, 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Every ghost cell at once.  With at least ng cells on every axis and no
+// hydrostatic face, the sequence of fills leaves in a ghost cell the value of one
+// interior cell, found axis by axis (each fill runs over the full transverse
+// extent, so a later one copies what an earlier one wrote), with the signs of the
+// axes' reflections multiplied.
+// ---------------------------------------------------------------------------
+struct GhostRule {
+  int direct;       // 0: the fills have to run one after another
+  int per[3];       // periodic axis
+  int type[3][2];   // FST_BC_* of the low / high face
+};
+
+inline GhostRule ghost_rule(const Geo& g, const fst_config& cf) {
+  GhostRule r{};
+  const int n[3] = {g.nci, g.ncj, g.nck};
+  const int per[3] = {cf.xper != 0, cf.yper != 0, cf.zper != 0};
+  const int t[3][2] = {{cf.bc_xmin, cf.bc_xmax}, {cf.bc_ymin, cf.bc_ymax}, {cf.bc_zmin, cf.bc_zmax}};
+  r.direct = 1;
+  for (int a = 0; a < g.ndim; ++a) {
+    r.per[a] = per[a];
+    for (int s = 0; s < 2; ++s) {
+      r.type[a][s] = t[a][s];
+      if (!per[a] && t[a][s] == FST_BC_HYDROSTATIC) r.direct = 0;
+    }
+    if (n[a] < g.ng) r.direct = 0;
+  }
+  return r;
+}
+
+// The interior cell behind ghost cell (i, j, k), in place, and the variables
+// 0..2 whose sign it takes flipped (bit v).
+__device__ __forceinline__ unsigned ghost_source(const Geo& g, const GhostRule& r, int& i, int& j,
+                                                 int& k) {
+  unsigned flip = 0;
+  auto axis = [&](int a, int& x, int n) {
+    const int side = x < g.ng ? 0 : x >= g.ng + n ? 1 : -1;
+    if (side < 0) return;
+    if (r.per[a]) {
+      x += side ? -n : n;
+      return;
+    }
+    x = side ? 2 * (g.ng + n) - 1 - x : 2 * g.ng - 1 - x;
+    const int t = r.type[a][side];
+    flip ^= t == FST_BC_NOSLIP ? 7u : t == FST_BC_REFLECTIVE ? 1u << a : 0u;
+  };
+  axis(0, i, g.nci);
+  axis(1, j, g.ncj);
+  if (g.ndim == 3) axis(2, k, g.nck);
+  return flip;
+}
+// x, its sign flipped when bit v of flip is set (what multiplying by -1 gives)
+__device__ __forceinline__ double ghost_value(double x, unsigned flip, int v) {
+  const unsigned long long b = fst64::bits_of(x);
+  return fst64::of_bits(v < 3 && ((flip >> v) & 1) ? b ^ 0x8000000000000000ull : b);
+}
+
 }  // namespace fstbc

@@ -7,6 +7,7 @@
 #include <string>
 #include <vector>
 
+#include "fst_bc_dev.cuh"
 #include "fst_common.cuh"
 
 // Optional CUDA-event bracketing of kernel launches (fst_set_profiling).
@@ -173,6 +174,11 @@ struct MixedBufs {
   const double* fused_for;
   // set by fst_rk_step_get_state for the final stage only
   MixedDownload* dl;
+  // set for a fused stage whose input's ghost cells are still to be filled: the
+  // shell pass then takes them from the interior (rule.direct); fill_state: and
+  // writes them to the state
+  bool fill, fill_state;
+  fstbc::GhostRule rule;
 };
 // exchange the current primitive set with b.alt
 void fst_mixed_swap(MixedBufs& b);

@@ -93,6 +93,51 @@ __global__ void __launch_bounds__(256) k_mprim3_shell(Geo g, Geo gq, Phys P,
   mprim3_cell<NS>(g, gq, P, U, O, false, i, j, k, lS, lC);
 }
 
+// The same with the boundary fill: the state values of a ghost cell come from the
+// interior cell behind it (fstbc::ghost_source) and go to U as well when
+// `store`.  One launch in place of the fills and k_mprim3_shell: the ghost values
+// are not written and read back in between.  Thread 0 resets the reduction words
+// the stage accumulates into.
+template <int NS>
+__global__ void __launch_bounds__(128) k_mfill3_shell(Geo g, Geo gq, Phys P, fstbc::GhostRule rule,
+                                                      double* U, int store, Prim3Out O, int nshell,
+                                                      unsigned long long* __restrict__ red) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t == 0) red[0] = red[1] = FST_KEY_LOWEST;
+  if (t >= nshell) return;
+  int i, j, k;
+  fst_shell_cell(g, t, i, j, k);
+  const long long sv = g.sv;
+  const long long dst = (long long)i + g.sy * j + g.sz * k;
+  const long long q = (long long)i + gq.sy * j + gq.sz * k;
+  const unsigned flip = fstbc::ghost_source(g, rule, i, j, k);
+  const long long src = (long long)i + g.sy * j + g.sz * k;
+  const bool ceq = g.nvt > g.nv;
+  double us[NS], um[4], uc[5];
+#pragma unroll
+  for (int d = 0; d < 4; ++d) um[d] = U[src + sv * d];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) us[s] = U[src + sv * (4 + s)];
+  if (ceq) {
+#pragma unroll
+    for (int n = 0; n < 5; ++n) uc[n] = U[src + sv * (g.nv + n)];
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) um[d] = fstbc::ghost_value(um[d], flip, d);
+  if (store) {
+#pragma unroll
+    for (int d = 0; d < 4; ++d) U[dst + sv * d] = um[d];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) U[dst + sv * (4 + s)] = us[s];
+    if (ceq) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) U[dst + sv * (g.nv + n)] = uc[n];
+    }
+  }
+  float lS = 0.f, lC = 0.f;
+  mprim3_vals<NS>(g, P, us, um, uc, O, q, gq.sv, false, 0, 0, 0, lS, lC);
+}
+
 // Fused upload: one thread per cell in storage order (as k_mprim3).  Every
 // state value comes from host memory over the host link and goes to U; the
 // interior cells also take mprim3_vals into the current primitive set.
@@ -209,6 +254,22 @@ void launch_mprim3(const Geo& g, const Phys& P, const MixedBufs& b, const double
     case 4: k_mprim3<4><<<qg, qb, 0, st>>>(g, b.gq, P, U, O, red); break;
     case 5: k_mprim3<5><<<qg, qb, 0, st>>>(g, b.gq, P, U, O, red); break;
     default: k_mprim3<0><<<qg, qb, 0, st>>>(g, b.gq, P, U, O, red); break;
+  }
+}
+
+// k_mfill3_shell (fused stages: up to 5 species)
+void launch_mfill3(const Geo& g, const Phys& P, const MixedBufs& b, double* U, cudaStream_t st) {
+  const Prim3Out O = prim3_out(P, b, false);
+  const int shell = (int)fst_shell_count(g);
+  const unsigned nb = cdiv(shell, 128);
+  switch (g.ns) {
+#define FST_FILL(N)                                                                         \
+  case N:                                                                                   \
+    k_mfill3_shell<N><<<nb, 128, 0, st>>>(g, b.gq, P, b.rule, U, b.fill_state, O, shell,   \
+                                          b.alt.red);                                       \
+    break;
+    FST_FILL(1) FST_FILL(2) FST_FILL(3) FST_FILL(4) FST_FILL(5)
+#undef FST_FILL
   }
 }
 
@@ -360,13 +421,16 @@ int fst_mixed_stage(const Geo& g, const Phys& P, const fst_config& cf, MixedBufs
     fst_fill_keys(b.red, 2, FST_KEY_LOWEST, st);
     ++n;
   }
-  if (fuse) {
+  const bool fill = have && b.fill;  // the shell pass fills the ghosts and resets the words
+  if (fuse && !fill) {
     fst_fill_keys(b.alt.red, 2, FST_KEY_LOWEST, st);
     ++n;
   }
   const MixedView M{b.Q, b.rho32, b.vel32, b.p64,  b.mu32,
                     b.nrg, b.C, b.T32, b.rho64, b.p32, b.plo};
-  if (g.ndim == 3 && have) {
+  if (fill) {
+    FST_LAUNCH(prof, "mfill3d_shell", st, n, launch_mfill3(g, P, b, const_cast<double*>(Uin), st));
+  } else if (g.ndim == 3 && have) {
     FST_LAUNCH(prof, "mprim3d_shell", st, n, launch_mprim3(g, P, b, Uin, false, nullptr, st, true));
   } else if (g.ndim == 3) {
     FST_LAUNCH(prof, "mprim3d", st, n,
