@@ -161,18 +161,18 @@ void setup_phys(const fst_config& cf, const Geo& g, Phys& P) {
   // 2D: dz = dx (src/input.cpp:402); the generalized 3D module passes cf.dx as
   // the z spacing of its fluxes (src/gen3d.cpp:359), its only use of dz
   P.dz = g.ndim == 3 && cart ? cf.dz : cf.dx;
-  P.ddx = make_div(P.dx);
-  P.ddy = make_div(P.dy);
-  P.ddz = make_div(P.dz);
-  P.d4x = make_div(4 * P.dx);
-  P.d4y = make_div(4 * P.dy);
-  P.d4z = make_div(4 * P.dz);
-  P.d12x = make_div(12.0 * P.dx);
-  P.d12y = make_div(12.0 * P.dy);
-  P.d12z = make_div(12.0 * P.dz);
+  P.dd[0] = make_div(P.dx);
+  P.dd[1] = make_div(P.dy);
+  P.dd[2] = make_div(P.dz);
+  P.d4[0] = make_div(4 * P.dx);
+  P.d4[1] = make_div(4 * P.dy);
+  P.d4[2] = make_div(4 * P.dz);
+  P.d12[0] = make_div(12.0 * P.dx);
+  P.d12[1] = make_div(12.0 * P.dy);
+  P.d12[2] = make_div(12.0 * P.dz);
   P.d12pz = make_div(12.0 * P.dy);
-  P.r12x = 1.0 / P.d12x.d;
-  P.r12y = 1.0 / P.d12y.d;
+  P.r12x = 1.0 / P.d12[0].d;
+  P.r12y = 1.0 / P.d12[1].d;
   P.r12pz = 1.0 / P.d12pz.d;
   P.dt = cf.dt;
   P.hdt = 0.5f * cf.dt;
@@ -193,9 +193,9 @@ void setup_phys(const fst_config& cf, const Geo& g, Phys& P) {
   P.rd_f[0] = (float)(1.0 / P.dx);
   P.rd_f[1] = (float)(1.0 / P.dy);
   P.rd_f[2] = (float)(1.0 / P.dz);
-  P.r12_f[0] = (float)(1.0 / P.d12x.d);
-  P.r12_f[1] = (float)(1.0 / P.d12y.d);
-  P.r12_f[2] = (float)(1.0 / P.d12z.d);
+  P.r12_f[0] = (float)(1.0 / P.d12[0].d);
+  P.r12_f[1] = (float)(1.0 / P.d12[1].d);
+  P.r12_f[2] = (float)(1.0 / P.d12[2].d);
   P.dxmag_f = (float)P.dxmag;
   P.dxmag2_f = (float)P.dxmag2;
   P.eps_f = (float)P.eps;

@@ -31,6 +31,10 @@ struct DivC {
   __device__ __forceinline__ double operator()(double a) const {
     return inv != 0.0 ? fst64::scale2(a, k, inv) : fst64::div_by(a, r);
   }
+  // the same with the division as a call (fst64::div_call)
+  __device__ __forceinline__ double call(double a) const {
+    return inv != 0.0 ? fst64::scale2(a, k, inv) : fst64::div_call(a, r.hi, r.lo, r.R);
+  }
 };
 
 // Physics constants of one run, passed by value to the kernels.
@@ -45,10 +49,10 @@ struct Phys {
   // (src/ceq.hpp:61-66): gammas = cd(6+2s), Rs = cd(7+2s)
   double cp2_s[FST_MAX_SPECIES], cv2_s[FST_MAX_SPECIES];
   double dx, dy, dz;
-  DivC ddx, ddy, ddz;     // x/dx, x/dy, x/dz
-  DivC d4x, d4y, d4z;     // x/(4*dx) ... (viscous and C-equation tangential terms)
-  DivC d12x, d12y, d12z;  // x/(12.0*dx) ... (4th-order derivatives)
-  DivC d12pz;             // x/(12.0*cd(2)): the reference's dz = cd(2) in presgrad3D
+  DivC dd[3];             // a/dx, a/dy, a/dz
+  DivC d4[3];             // a/(4*dx) ... (viscous and C-equation tangential terms)
+  DivC d12[3];            // a/(12.0*dx) ... (4th-order derivatives)
+  DivC d12pz;             // a/(12.0*cd(2)): the reference's dz = cd(2) in presgrad3D
   double r12x, r12y, r12pz;  // their reciprocals (mixed path)
   double dt, hdt;         // dt and 0.5f*dt
   double kap, eps, alpha, g, rho_ref;
@@ -95,6 +99,40 @@ __host__ __device__ __forceinline__ double fst_unkey(unsigned long long k) {
 }
 // Kokkos::Max starts from -DBL_MAX and `if (s > lmax)` never takes a NaN.
 #define FST_KEY_LOWEST 0x0010000000000000ull /* fst_key(-DBL_MAX) */
+
+// Running maximum on the order-preserving key, NaN skipped: integer work, where
+// FP64 compares would each take the FP64 unit's time.
+__device__ __forceinline__ void fst_key_max(unsigned long long& k, double x) {
+  const unsigned long long b = fst64::bits_of(x);
+  if ((b & 0x7FFFFFFFFFFFFFFFull) > 0x7FF0000000000000ull) return;
+  const unsigned long long q = (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+  k = q > k ? q : k;
+}
+// The maxima of two keys over a block of 32 W threads (every thread calls it) into
+// word[0] and word[1]: one atomic per block and word.
+template <int W>
+__device__ __forceinline__ void fst_key_max_block(unsigned long long* word, unsigned long long a,
+                                                  unsigned long long b) {
+  __shared__ unsigned long long sa[W], sb[W];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long x = __shfl_xor_sync(0xffffffffu, a, o);
+    const unsigned long long y = __shfl_xor_sync(0xffffffffu, b, o);
+    a = x > a ? x : a;
+    b = y > b ? y : b;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sa[threadIdx.x >> 5] = a;
+    sb[threadIdx.x >> 5] = b;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const unsigned long long* s = threadIdx.x ? sb : sa;
+    unsigned long long m = s[0];
+    for (int w = 1; w < W; ++w) m = s[w] > m ? s[w] : m;
+    atomicMax(&word[threadIdx.x], m);
+  }
+}
 
 // Warp-wide max of per-thread maxima that already skipped NaN.
 __device__ __forceinline__ double fst_warp_max(double v) {

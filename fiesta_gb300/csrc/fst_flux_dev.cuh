@@ -280,7 +280,7 @@ inline Plan make_plan(const Geo& g, const Phys& P) {
   p.ndim = g.ndim;
   const int n[3] = {g.nci, g.ncj, g.nck};
   const long long s[3] = {1, g.sy, g.sz};
-  const DivC dd[3] = {P.ddx, P.ddy, P.ddz};
+  const DivC dd[3] = {P.dd[0], P.dd[1], P.dd[2]};
   const long long base = g.ng + g.sy * g.ng + (g.ndim == 3 ? g.sz * g.ng : 0);
   long long chunks = 0;  // 32-line chunks per face layer, all directions
   for (int d = 0; d < g.ndim; ++d) {

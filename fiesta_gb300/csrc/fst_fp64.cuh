@@ -91,11 +91,14 @@ FST_HD uint32_t bits_of_f(float f) {
 #endif
 }
 
-// the operator, out of line: the rare operands' path
+// The rare operands' path, out of line: inlined, the operator would be predicated
+// or run ahead of the test and take the FP64 unit's time for every operand.
 #if defined(__CUDACC__)
 __host__ __device__ __noinline__ static double div_any(double a, double b) { return a / b; }
+__host__ __device__ __noinline__ static double mul_any(double a, double b) { return a * b; }
 #else
 inline double div_any(double a, double b) { return a / b; }
+inline double mul_any(double a, double b) { return a * b; }
 #endif
 
 // R with R / 2^32 = 1/b' (1 - e), |e| < 2^-30, for the divisor mantissa b' = B
@@ -180,9 +183,12 @@ FST_HD double scale2(double a, int k, double p) {
   const uint32_t hi = (uint32_t)(ba >> 32);
   const uint32_t e = (hi >> 20) & 0x7FFu;
   const bool zero = (ba << 1) == 0;
-  if (!zero && (e - 1u >= 2046u || e + (uint32_t)k - 1u >= 2046u)) return a * p;
+  if (!zero && (e - 1u >= 2046u || e + (uint32_t)k - 1u >= 2046u)) return mul_any(a, p);
   return of_bits(((uint64_t)(hi + (zero ? 0u : (uint32_t)k << 20)) << 32) | (uint32_t)ba);
 }
+FST_HD double half(double a) { return scale2(a, -1, 0.5); }
+FST_HD double twice(double a) { return scale2(a, 1, 2.0); }
+FST_HD double eight(double a) { return scale2(a, 3, 8.0); }
 
 #if defined(__CUDACC__)
 // ---------------------------------------------------------------------------
@@ -338,5 +344,36 @@ FST_HD double div_const(double b) {
       quot55((uint32_t)(k.m >> 32), (uint32_t)k.m, bh, y.l, recip32(bh, y.l));
   return of_bits(round_quot(q, ((2044u + (uint32_t)k.e) << 20) - (y.h & 0x7FF00000u), 0));
 }
+
+
+// a b rounded as IEEE for every input: the integer product where both are normal
+// (or one is zero and the other normal or zero) and the result is normal, the
+// operator elsewhere.
+FST_HD double mul_rn(double a, double b) {
+  const W2 x = words(a), y = words(b);
+  const uint32_t ex = (x.h >> 20) & 0x7FFu, ey = (y.h >> 20) & 0x7FFu;
+  const bool zx = ((x.h << 1) | x.l) == 0, zy = ((y.h << 1) | y.l) == 0, zero = zx || zy;
+  const uint32_t sg = (x.h ^ y.h) & 0x80000000u;
+  if ((!zx && ex - 1u >= 2046u) || (!zy && ey - 1u >= 2046u) ||
+      (!zero && ex + ey - 1025u >= 2044u))
+    return mul_any(a, b);
+  const uint32_t xh = mant_hi(x.h), yh = mant_hi(y.h);
+  const uint64_t ll = (uint64_t)x.l * y.l;
+  const uint64_t m1 = (uint64_t)xh * y.l + (ll >> 32);
+  const uint64_t m2 = (uint64_t)x.l * yh + (uint32_t)m1;
+  const uint64_t H = (uint64_t)xh * yh + (m1 >> 32) + (m2 >> 32);
+  const uint64_t r = round_product(H, (uint32_t)m2, (uint32_t)ll, (ex + ey - 1024u) << 20, sg);
+  return of_bits(zero ? (uint64_t)sg << 32 : r);
+}
+
+#if defined(__CUDACC__)
+// mul_rn, div_by and a/d as calls, for long straight-line kernels: inlined, a
+// few dozen of them overflow the instruction caches, and the warps wait for
+// instructions more than for anything else.
+__device__ __noinline__ static double mul_call(double a, double b) { return mul_rn(a, b); }
+__device__ __noinline__ static double div_call(double a, uint32_t hi, uint32_t lo, uint32_t R) {
+  return div_by(a, Recip{hi, lo, R});
+}
+#endif
 
 }  // namespace fst64

@@ -22,6 +22,11 @@
 namespace {
 using fst64::div_by;
 using fst64::div_rn;
+using fst64::eight;
+using fst64::half;
+using fst64::mul_call;
+using fst64::mul_rn;
+using fst64::twice;
 
 // calculateRhoPT2D (src/secondary.hpp:60-107), computeVelocity2D
 // (src/velocity.hpp:85-99); maxWaveSpeed2D and maxCvar2D(var, 1)
@@ -34,59 +39,55 @@ __global__ void __launch_bounds__(256) k_prim2d(Geo g, Phys P, const double* __r
                                                 const double* __restrict__ met) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long sv = g.sv;
-  double lS = -1.7976931348623157e308, lC = -1.7976931348623157e308;
+  const fst64::Fused k(P.ns);
+  unsigned long long kS = FST_KEY_LOWEST, kC = FST_KEY_LOWEST;
   if (c < sv) {
     double r = 0.0;
-    for (int s = 0; s < P.ns; ++s) r = r + U[c + sv * (3 + s)];
+    for (int s = 0; s < P.ns; ++s) r = k.add(r, U[c + sv * (3 + s)]);
     const fst64::Recip rr = fst64::recip_of(r);
     double Cp = 0, Cv = 0, Cp2 = 0, Cv2 = 0;
     for (int s = 0; s < P.ns; ++s) {
       double ys = div_by(U[c + sv * (3 + s)], rr);
-      Cp = Cp + ys * P.cp_s[s];
-      Cv = Cv + ys * P.cv_s[s];
+      Cp = k.add(Cp, mul_rn(ys, P.cp_s[s]));
+      Cv = k.add(Cv, mul_rn(ys, P.cv_s[s]));
       if (red) {
-        Cp2 = Cp2 + ys * P.cp2_s[s];
-        Cv2 = Cv2 + ys * P.cv2_s[s];
+        Cp2 = k.add(Cp2, mul_rn(ys, P.cp2_s[s]));
+        Cv2 = k.add(Cv2, mul_rn(ys, P.cv2_s[s]));
       }
     }
     const double gam = div_rn(Cp, Cv);
     const double m0 = U[c], m1 = U[c + sv], E = U[c + 2 * sv];
-    const double p = (gam - 1) * (E - div_by(0.5, rr) * (m0 * m0 + m1 * m1));
+    const double mm = k.add(mul_rn(m0, m0), mul_rn(m1, m1));
+    const double p = mul_rn(k.sub(gam, 1.0), k.sub(E, mul_rn(div_by(0.5, rr), mm)));
     const double u = div_by(m0, rr), v = div_by(m1, rr);
     rho[c] = r;
     pr[c] = p;
     if (met) {
       // computeGenVelocity2D (src/velocity.hpp:49-66), metric (a,b) at
       // met[c + sv*(a + 2b)]
-      vel[c] = div_by(met[c] * m0, rr) + div_by(met[c + 2 * sv] * m1, rr);
-      vel[c + sv] = div_by(met[c + sv] * m0, rr) + div_by(met[c + 3 * sv] * m1, rr);
+      vel[c] = k.add(div_by(mul_rn(met[c], m0), rr), div_by(mul_rn(met[c + 2 * sv], m1), rr));
+      vel[c + sv] =
+          k.add(div_by(mul_rn(met[c + sv], m0), rr), div_by(mul_rn(met[c + 3 * sv], m1), rr));
     } else {
       vel[c] = u;
       vel[c + sv] = v;
     }
-    if (T) T[c] = div_rn(p, (Cp - Cv) * r);
-    if (nrg) nrg[c] = div_by(E, rr) - 0.5 * r * (u * u + v * v);
+    if (T) T[c] = div_rn(p, mul_rn(k.sub(Cp, Cv), r));
+    if (nrg) nrg[c] = k.sub(div_by(E, rr),
+                           mul_rn(half(r), k.add(mul_rn(u, u), mul_rn(v, v))));
     if (red) {
       int i = (int)(c % g.sy), j = (int)(c / g.sy);
       bool in = i >= g.ng && i < g.ngi - g.ng && j >= g.ng && j < g.ngj - g.ng;
       if (in) {
         const double gam2 = div_rn(Cp2, Cv2);
-        double a = sqrt(div_by(gam2 * p, rr));
-        double s = a + sqrt(m0 * m0 + m1 * m1);
-        if (s > lS) lS = s;
-        double ch = fabs(U[c + sv * (P.nv + 1)]);
-        if (ch > lC) lC = ch;
+        double a = sqrt(div_by(mul_rn(gam2, p), rr));
+        double s = k.add(a, sqrt(mm));
+        fst_key_max(kS, s);
+        fst_key_max(kC, fabs(U[c + sv * (P.nv + 1)]));
       }
     }
   }
-  if (red) {
-    lS = fst_warp_max(lS);
-    lC = fst_warp_max(lC);
-    if ((threadIdx.x & 31) == 0) {
-      atomicMax(&red[0], fst_key(lS));
-      atomicMax(&red[1], fst_key(lC));
-    }
-  }
+  if (red) fst_key_max_block<8>(red, kS, kC);
 }
 
 // The centred and QUICK schemes (computeFluxCentered2D / computeFluxQuick2D,
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __r
                  12.0);
       const double pf =
           div_rn(0.0 - pr[c + 2 * s] + 7.0 * pr[c + s] + 7.0 * pr[c] - pr[c - s], 12.0);
-      const DivC dd = dir == 0 ? P.ddx : P.ddy;
+      const DivC dd = dir == 0 ? P.dd[0] : P.dd[1];
       double* Fd = F + (long long)dir * P.nv * sv;
 #pragma unroll 1
       for (int v = 0; v < P.nv; ++v) {
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __r
     const double* vd = vel + sv * dir;
     const double uf =
         div_rn(-vd[c + 2 * s] + 7.0 * vd[c + s] + 7.0 * vd[c] - vd[c - s], 12.0);
-    const DivC dd = dir == 0 ? P.ddx : P.ddy;
+    const DivC dd = dir == 0 ? P.dd[0] : P.dd[1];
     double* Fd = F + (long long)dir * P.nv * sv;
 #pragma unroll 1
     for (int v = 0; v < P.nv; ++v) {
@@ -155,10 +156,64 @@ __global__ void __launch_bounds__(128) k_flux2d(Geo g, Phys P, const double* __r
 }
 
 // calculateStressTensor2dv + calculateHeatFlux2dv (src/viscosity.hpp:25-136)
-// and computeCeqFlux2D * computeCeqFaces2D (src/ceq.hpp:200-267) on the x and
-// y faces of each face index.
-// S[(f*3 + {0:xx,1:xy,2:yy})*sv + cell], Q[f*sv + cell],
-// MF[((f*2+d)*2+w)*sv + cell].
+// and computeCeqFlux2D * computeCeqFaces2D (src/ceq.hpp:200-267) on the faces
+// with normal F of each face index (blockIdx.z = F).  Only the stress components
+// the momenta take on that face are formed.
+// S[(F*3 + {0:xx,1:xy,2:yy})*sv + cell], Q[F*sv + cell],
+// MF[((F*2+d)*2+w)*sv + cell].
+template <int F>
+__device__ __forceinline__ void face_terms2d(const Geo& g, const Phys& P, const fst64::Fused& k,
+                                             long long c, const double* __restrict__ U,
+                                             const double* __restrict__ rho,
+                                             const double* __restrict__ vel,
+                                             const double* __restrict__ T,
+                                             const unsigned long long* __restrict__ red,
+                                             double* __restrict__ S, double* __restrict__ Q,
+                                             double* __restrict__ MF) {
+  constexpr int A = 1 - F;
+  const long long sv = g.sv;
+  const long long sf = F == 0 ? 1 : g.sy, st = F == 0 ? g.sy : 1;
+  double G[2][2], tm[2];  // G[d][w]; tm[w]: the lower pair's sum of the tangential difference
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    const double* u = vel + sv * w;
+    G[F][w] = P.dd[F](k.sub(u[c + sf], u[c]));
+    tm[w] = k.add(u[c - st], u[c + sf - st]);
+    G[A][w] = P.d4[A](k.sub(k.add(u[c + st], u[c + sf + st]), tm[w]));
+  }
+  if (P.visc) {
+    const double mu = P.mu2d;
+    double dudy = G[1][0];
+    // the reference's vel(i,j-1,1) in du/dy on the x faces (src/viscosity.hpp:68)
+    if (F == 0)
+      dudy = P.d4[1](k.sub(k.add(vel[c + st], vel[c + sf + st]),
+                           k.add(vel[c + sv - st], vel[c + sf - st])));
+    const double n = F == 0 ? k.sub(twice(G[0][0]), G[1][1]) : k.sub(twice(G[1][1]), G[0][0]);
+    S[(long long)(F * 3 + 2 * F) * sv + c] = mul_call((2.0 / 3.0) * mu, n);
+    S[(long long)(F * 3 + 1) * sv + c] = mul_call(mu, k.add(dudy, G[0][1]));
+    Q[F * sv + c] = P.dd[F](mul_call(-P.kheat2d, k.sub(T[c + sf], T[c])));
+  }
+  if (P.ceq) {
+    const double* C = U + sv * P.nv;
+    const double maxCh = fst_unkey(red[1]);
+    const double alpha = mul_call(div_rn(P.dxmag2, k.add(maxCh, 1.0e-6)), P.alpha);  // src/cart2d.cpp:227
+    auto mean = [&](const double* a) { return half(k.add(a[c], a[c + sf])); };
+    const double ar = mul_call(mul_call(alpha, mean(rho)), mean(C + sv));
+    const double ct[2] = {mean(C + 2 * sv), mean(C + 3 * sv)};
+    const double own = mul_call(ct[F], ct[F]), other = mul_call(ct[A], ct[A]);
+    const double ctmag = k.add(F == 0 ? k.add(own, other) : k.add(other, own), 1.0e-6);
+    const fst64::Recip rmag = fst64::recip_of(ctmag);
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      const double cc = d == F ? own : mul_call(ct[F], ct[d]);
+      const double m = fst64::div_call(mul_call(ar, cc), rmag.hi, rmag.lo, rmag.R);
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        MF[(long long)((F * 2 + d) * 2 + w) * sv + c] = k.mul(m, G[d][w]);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __restrict__ U,
                                                  const double* __restrict__ rho,
                                                  const double* __restrict__ vel,
@@ -170,70 +225,15 @@ __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __
   const int j = g.ng - 1 + blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= g.ngi - g.ng || j >= g.ngj - g.ng) return;
   const long long c = fst_idx(g, i, j, 0);
-  const long long sv = g.sv, sx = 1, sy = g.sy;
-  const double* u = vel;
-  const double* v = vel + sv;
-  if (P.visc) {
-    const double mu = P.mu2d;
-    double dudx, dvdy, dudy, dvdx;
-    // x face
-    dudx = P.ddx(u[c + sx] - u[c]);
-    dvdx = P.ddx(v[c + sx] - v[c]);
-    dudy = P.d4y((u[c + sy] + u[c + sx + sy]) - (v[c - sy] + u[c + sx - sy]));
-    dvdy = P.d4y((v[c + sy] + v[c + sx + sy]) - (v[c - sy] + v[c + sx - sy]));
-    S[0 * sv + c] = (2.0 / 3.0) * mu * (2.0 * dudx - dvdy);
-    S[2 * sv + c] = (2.0 / 3.0) * mu * (2.0 * dvdy - dudx);
-    S[1 * sv + c] = mu * (dudy + dvdx);
-    // y face
-    dudx = P.d4x((u[c + sx] + u[c + sx + sy]) - (u[c - sx] + u[c - sx + sy]));
-    dvdx = P.d4x((v[c + sx] + v[c + sx + sy]) - (v[c - sx] + v[c - sx + sy]));
-    dudy = P.ddy(u[c + sy] - u[c]);
-    dvdy = P.ddy(v[c + sy] - v[c]);
-    S[3 * sv + c] = (2.0 / 3.0) * mu * (2.0 * dudx - dvdy);
-    S[5 * sv + c] = (2.0 / 3.0) * mu * (2.0 * dvdy - dudx);
-    S[4 * sv + c] = mu * (dudy + dvdx);
-    // heat flux
-    Q[c] = P.ddx(-P.kheat2d * (T[c + sx] - T[c]));
-    Q[sv + c] = P.ddy(-P.kheat2d * (T[c + sy] - T[c]));
-  }
-  if (P.ceq) {
-    const int nv = P.nv;
-    const double maxCh = fst_unkey(red[1]);
-    const double alpha = div_rn(P.dxmag2, maxCh + 1.0e-6) * P.alpha;  // src/cart2d.cpp:227
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-      const long long sf = f == 0 ? sx : sy;
-      const double r = (rho[c] + rho[c + sf]) / 2.0;
-      const double chat = (U[c + sv * (nv + 1)] + U[c + sf + sv * (nv + 1)]) / 2.0;
-      double ct[2];
-      ct[0] = (U[c + sv * (nv + 2)] + U[c + sf + sv * (nv + 2)]) / 2.0;
-      ct[1] = (U[c + sv * (nv + 3)] + U[c + sf + sv * (nv + 3)]) / 2.0;
-      const double ctmag = (ct[0] * ct[0] + ct[1] * ct[1]) + 1.0e-6;
-      const fst64::Recip rmag = fst64::recip_of(ctmag);
-#pragma unroll
-      for (int w = 0; w < 2; ++w) {
-        const double* vw = vel + sv * w;
-        double gr[2];
-        if (f == 0) {
-          gr[0] = P.ddx(vw[c + sx] - vw[c]);
-          gr[1] = P.d4y((vw[c + sy] + vw[c + sx + sy]) - (vw[c - sy] + vw[c + sx - sy]));
-        } else {
-          gr[0] = P.d4x((vw[c + sx] + vw[c + sx + sy]) - (vw[c - sx] + vw[c - sx + sy]));
-          gr[1] = P.ddy(vw[c + sy] - vw[c]);
-        }
-#pragma unroll
-        for (int d = 0; d < 2; ++d) {
-          const double m = div_by(alpha * r * chat * (ct[f] * ct[d]), rmag);
-          MF[(long long)((f * 2 + d) * 2 + w) * sv + c] = m * gr[d];
-        }
-      }
-    }
-  }
+  const fst64::Fused k(P.nv);
+  if (blockIdx.z == 0) face_terms2d<0>(g, P, k, c, U, rho, vel, T, red, S, Q, MF);
+  else face_terms2d<1>(g, P, k, c, U, rho, vel, T, red, S, Q, MF);
 }
 
 // Per interior cell: advect2D, applyPressureGradient2D, computeBuoyancy,
 // applyViscousTerm2dv, calculateRhoGrad2D, updateCeq2D, applyCeq2D, then the
-// stage combine (src/rk.cpp:42-69).
+// stage combine (src/rk.cpp:42-69).  blockIdx.z: 0 the momenta and energy, 1 the
+// species, 2 the C variables, which share nothing.
 __global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __restrict__ U,
                                                 const double* __restrict__ rho,
                                                 const double* __restrict__ pr,
@@ -253,117 +253,131 @@ __global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __r
   const long long c = fst_idx(g, i, j, 0);
   const long long sv = g.sv, sx = 1, sy = g.sy;
   const int nv = P.nv;
+  const fst64::Fused k(nv);
   auto emit = [&](int v, double R) {
     if (Rout) Rout[c + sv * v] = R;
-    else Unew[c + sv * v] = Uold[c + sv * v] + coef * R;
+    else Unew[c + sv * v] = k.add(Uold[c + sv * v], mul_call(coef, R));
   };
   auto divF = [&](int v) {
     const double* Fx = F + sv * v;
     const double* Fy = F + sv * (nv + v);
-    return -((Fx[c] - Fx[c - sx]) + (Fy[c] - Fy[c - sy]));
+    return -k.add(k.sub(Fx[c], Fx[c - sx]), k.sub(Fy[c], Fy[c - sy]));
   };
+  // ((a- - 8 b-) + 8 b+) - a+ of the four neighbours along a direction
+  auto d4sum = [&](double am, double bm, double bp, double ap) {
+    return k.sub(k.add(k.sub(am, eight(bm)), eight(bp)), ap);
+  };
+  if (blockIdx.z == 1) {
+    for (int v = 3; v < nv; ++v) emit(v, divF(v));
+    // C-equation variables carried without a right-hand side (the generalized
+    // module evolves none): U + coef*0, as the reference's zero dvar gives
+    if (!P.ceq)
+      for (int v = nv; v < g.nvt; ++v) emit(v, 0.0);
+    return;
+  }
+  if (blockIdx.z == 2) {
+    auto d4 = [&](const double* a, int f) {
+      const long long s = f == 0 ? sx : sy;
+      return P.d12[f].call(d4sum(a[c - 2 * s], a[c - s], a[c + s], a[c + 2 * s]));
+    };
+    const double dxr = d4(rho, 0), dyr = d4(rho, 1);
+    const double dxe = d4(nrg, 0), dye = d4(nrg, 1);
+    const double dxu = d4(vel, 0), dyv = d4(vel + sv, 1);
+    const double g2 = k.add(mul_call(dxr, dxr), mul_call(dyr, dyr));
+    const double rgrad = sqrt(g2);
+    const double divu = k.add(dxu, dyv);
+    const double dnednr = mul_call(k.add(mul_call(dxr, dxe), mul_call(dyr, dye)), g2);
+    // (1 - i1) i2 rgrad and i1 rgrad of the reference: the factors are 0 or 1
+    const bool i1 = dnednr < 0.0, i2 = divu < 0.0;
+    const double maxS = fst_unkey(red[0]);
+    const double src = div_rn(maxS, P.eps * P.dxmag);
+    const double dif = P.kap * maxS * P.dxmag;
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n) {
+      const double Gn = n == 0   ? mul_call(!i1 && i2 ? 1.0 : 0.0, rgrad)
+                        : n == 1 ? mul_call(i1 ? 1.0 : 0.0, rgrad)
+                        : n == 2 ? -dyr
+                                 : dxr;
+      const double* Cn = U + sv * (nv + n);
+      const double cc = Cn[c];
+      const double dx_right = P.dd[0].call(k.sub(Cn[c + sx], cc));
+      const double dx_left = P.dd[0].call(k.sub(cc, Cn[c - sx]));
+      const double dy_top = P.dd[1].call(k.sub(Cn[c + sy], cc));
+      const double dy_bot = P.dd[1].call(k.sub(cc, Cn[c - sy]));
+      const double lap = k.sub(k.add(k.sub(dx_right, dx_left), dy_top), dy_bot);
+      emit(nv + n, k.add(mul_call(src, k.sub(Gn, cc)), mul_call(dif, lap)));
+    }
+    emit(nv + 4, 0.0);  // the fifth C variable has no right-hand side
+    return;
+  }
   double R0 = divF(0), R1 = divF(1), R2 = divF(2);
-  for (int v = 3; v < nv; ++v) emit(v, divF(v));
   if (met) {
     // applyGenPressureGradient2D (src/presgrad.hpp:148-190)
-    auto d4m = [&](long long st, int a, int w) {
+    auto d4m = [&](long long s, int a, int w) {
       const double* m = met + sv * (a + 2 * w);
-      return div_rn(pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
-                        8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st],
+      // 8.0 * p * m: the product with 8 first, exact
+      return div_rn(k.sub(k.add(k.sub(mul_call(pr[c - 2 * s], m[c - 2 * s]),
+                                      mul_call(eight(pr[c - s]), m[c - s])),
+                                mul_call(eight(pr[c + s]), m[c + s])),
+                          mul_call(pr[c + 2 * s], m[c + 2 * s])),
                     12.0);
     };
-    R0 = R0 - (d4m(sx, 0, 0) + d4m(sy, 1, 0));
-    R1 = R1 - (d4m(sx, 0, 1) + d4m(sy, 1, 1));
+    R0 = k.sub(R0, k.add(d4m(sx, 0, 0), d4m(sy, 1, 0)));
+    R1 = k.sub(R1, k.add(d4m(sx, 0, 1), d4m(sy, 1, 1)));
   } else {
-    const double dxp =
-        P.d12x(pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]);
-    const double dyp =
-        P.d12y(pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]);
-    R0 -= dxp;
-    R1 -= dyp;
+    R0 = k.sub(R0, P.d12[0].call(d4sum(pr[c - 2 * sx], pr[c - sx], pr[c + sx], pr[c + 2 * sx])));
+    R1 = k.sub(R1, P.d12[1].call(d4sum(pr[c - 2 * sy], pr[c - sy], pr[c + sy], pr[c + 2 * sy])));
   }
   if (P.buoyancy) {
     const double vb = div_rn(U[c + sv], U[c + 3 * sv]);
-    const double rhop = rho[c] - P.rho_ref;
+    const double rhop = k.sub(rho[c], P.rho_ref);
     const double eps = 1e-6;
     if (rhop >= eps || rhop <= -eps) {
-      const double f = -P.g * rhop;
-      R1 += f;
-      R2 += fabs(vb) * f;
+      const double f = mul_call(-P.g, rhop);
+      R1 = k.add(R1, f);
+      R2 = k.add(R2, mul_call(fabs(vb), f));
     }
   }
   if (P.visc) {
     const double* u = vel;
     const double* v = vel + sv;
-    const double ur = (u[c + sx] + u[c]) / 2.0, ul = (u[c - sx] + u[c]) / 2.0;
-    const double vr = (v[c + sx] + v[c]) / 2.0, vl = (v[c - sx] + v[c]) / 2.0;
-    const double ut = (u[c + sy] + u[c]) / 2.0, ub = (u[c - sy] + u[c]) / 2.0;
-    const double vt = (v[c + sy] + v[c]) / 2.0, vb = (v[c - sy] + v[c]) / 2.0;
+    auto mean = [&](const double* a, long long s) { return half(k.add(a[c + s], a[c])); };
     const double* sxx = S;
     const double* sxy = S + sv;
     const double* syx = S + 4 * sv;  // stressy(1,0) == stressy(0,1)
     const double* syy = S + 5 * sv;
-    const double a = P.ddx(sxx[c] - sxx[c - sx]) + P.ddy(syx[c] - syx[c - sy]);
-    const double b = P.ddx(sxy[c] - sxy[c - sx]) + P.ddy(syy[c] - syy[c - sy]);
-    const double c1 = P.ddx(ur * sxx[c] - ul * sxx[c - sx]) + P.ddx(vr * sxy[c] - vl * sxy[c - sx]) +
-                      P.ddy(ut * syx[c] - ub * syx[c - sy]) + P.ddy(vt * syy[c] - vb * syy[c - sy]);
-    const double c2 = P.ddx(Q[c] - Q[c - sx]) + P.ddy(Q[sv + c] - Q[sv + c - sy]);
-    R0 = R0 + a;
-    R1 = R1 + b;
-    R2 = R2 + c1 - c2;
+    auto diff = [&](const double* s, int f) {
+      return P.dd[f].call(k.sub(s[c], s[c - (f == 0 ? sx : sy)]));
+    };
+    // (a b)(face) - (a b)(face before) over the spacing
+    auto work = [&](const double* a, const double* s, int f) {
+      const long long st = f == 0 ? sx : sy;
+      return P.dd[f].call(
+          k.sub(mul_call(mean(a, st), s[c]), mul_call(mean(a, -st), s[c - st])));
+    };
+    const double a = k.add(diff(sxx, 0), diff(syx, 1));
+    const double b = k.add(diff(sxy, 0), diff(syy, 1));
+    const double c1 = k.add(k.add(k.add(work(u, sxx, 0), work(v, sxy, 0)), work(u, syx, 1)),
+                            work(v, syy, 1));
+    const double c2 = k.add(diff(Q, 0), diff(Q + sv, 1));
+    R0 = k.add(R0, a);
+    R1 = k.add(R1, b);
+    R2 = k.sub(k.add(R2, c1), c2);
   }
   if (P.ceq) {
-    auto d4 = [&](const double* a, long long st, const DivC& d12) {
-      return d12(a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]);
-    };
-    const double dxr = d4(rho, sx, P.d12x), dyr = d4(rho, sy, P.d12y);
-    const double dxe = d4(nrg, sx, P.d12x), dye = d4(nrg, sy, P.d12y);
-    const double dxu = d4(vel, sx, P.d12x), dyv = d4(vel + sv, sy, P.d12y);
-    const double n1 = dxr, n2 = dyr;
-    const double rgrad = sqrt(dxr * dxr + dyr * dyr);
-    const double divu = dxu + dyv;
-    const double dnednr = (n1 * dxe + n2 * dye) * (n1 * dxr + n2 * dyr);
-    const double i1 = dnednr < 0.0 ? 1.0 : 0.0;
-    const double i2 = divu < 0.0 ? 1.0 : 0.0;
-    double G[4];
-    G[0] = (1 - i1) * i2 * rgrad;
-    G[1] = i1 * rgrad;
-    G[2] = -dyr;
-    G[3] = dxr;
-    const double maxS = fst_unkey(red[0]);
-    const double src = div_rn(maxS, P.eps * P.dxmag);
-    const double dif = P.kap * maxS * P.dxmag;
-#pragma unroll
-    for (int n = 0; n < 4; ++n) {
-      const double* Cn = U + sv * (nv + n);
-      const double cc = Cn[c];
-      const double dx_right = P.ddx(Cn[c + sx] - cc);
-      const double dx_left = P.ddx(cc - Cn[c - sx]);
-      const double dy_top = P.ddy(Cn[c + sy] - cc);
-      const double dy_bot = P.ddy(cc - Cn[c - sy]);
-      const double lap = dx_right - dx_left + dy_top - dy_bot;
-      emit(nv + n, src * (G[n] - cc) + dif * lap);
-    }
-    emit(nv + 4, 0.0);  // the fifth C variable has no right-hand side
-#pragma unroll
+#pragma unroll 1
     for (int w = 0; w < 2; ++w) {
-      const double* m00 = MF + (long long)(0 * 2 + w) * sv;
-      const double* m01 = MF + (long long)(2 + w) * sv;
-      const double* m10 = MF + (long long)(4 + w) * sv;
-      const double* m11 = MF + (long long)(6 + w) * sv;
       double diffu = 0;
-      diffu += P.ddx(m00[c] - m00[c - sx]);
-      diffu += P.ddx(m01[c] - m01[c - sx]);
-      diffu += P.ddy(m10[c] - m10[c - sy]);
-      diffu += P.ddy(m11[c] - m11[c - sy]);
-      if (w == 0) R0 += diffu;
-      else R1 += diffu;
+#pragma unroll 1
+      for (int q = 0; q < 4; ++q) {  // (face, derivative) = (0,0), (0,1), (1,0), (1,1)
+        const double* m = MF + (long long)(2 * q + w) * sv;
+        const int f = q >> 1;
+        diffu = k.add(diffu, P.dd[f].call(k.sub(m[c], m[c - (f == 0 ? sx : sy)])));
+      }
+      if (w == 0) R0 = k.add(R0, diffu);
+      else R1 = k.add(R1, diffu);
     }
   }
-  // C-equation variables carried without a right-hand side (the generalized
-  // module evolves none): U + coef*0, as the reference's zero dvar gives
-  if (!P.ceq)
-    for (int v = nv; v < g.nvt; ++v) emit(v, 0.0);
   emit(0, R0);
   emit(1, R1);
   emit(2, R2);
@@ -407,9 +421,9 @@ int fst_plain2d_stage(const Geo& g, const Phys& P, const Plain2DBufs& b, const d
                k_flux2d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.F));
   if (P.visc || P.ceq) {
     FST_LAUNCH(prof, "faces2d", st, n,
-               k_faces2d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.T, b.red, b.S, b.Q, b.MF));
+               k_faces2d<<<dim3(gf.x, gf.y, 2), bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.T, b.red, b.S, b.Q, b.MF));
   }
-  const dim3 gc(cdiv(g.nci, 32), cdiv(g.ncj, 4), 1);
+  const dim3 gc(cdiv(g.nci, 32), cdiv(g.ncj, 4), P.ceq ? 3 : 2);
   FST_LAUNCH(prof, "cell2d", st, n,
              k_cell2d<<<gc, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.Q,
                                          b.MF, b.red, Uold, Unew, coef, Rout, b.met));

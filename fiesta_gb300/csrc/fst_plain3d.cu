@@ -10,9 +10,7 @@
 //   k_prim3d        rho, p, velocity, mass fractions, internal energy, and the
 //                   two global maxima of the C-equation (maxS, maxCh) folded
 //                   into the same pass (block max + one atomicMax per block)
-//   k_flux3d        WENO5 fluxes of all nv variables on the three faces
-//                   owned by each face index (each face computed once; the
-//                   face velocity computed once per face, not per variable)
+//   k_weno_flux     WENO5 fluxes of all nv variables (fst_flux_dev.cuh)
 //   k_faces3d       the 27 face velocity gradients, shared by the viscous
 //                   stress and the C-equation face terms, which are the same
 //                   expressions in the reference
@@ -21,7 +19,8 @@
 //                   RK stage combine straight into the next state buffer
 // On GB300 the FP64 pipe, not HBM, bounds this path, so the design removes
 // repeated FP64 work (species constants hoisted, Y_s and e computed once per
-// cell, shared gradients) while keeping every operation the reference
+// cell, shared gradients) and moves divisions and products to the integer pipes
+// (fst_fp64.cuh) while keeping the result of every operation the reference
 // performs on every value it stores, in the same order.  Built with
 // --fmad=false so no a*b+c is contracted: results match the reference's FP64
 // run bit for bit.
@@ -30,13 +29,22 @@
 namespace {
 using fst64::div_by;
 using fst64::div_rn;
+using fst64::eight;
+using fst64::half;
+using fst64::mul_call;
+using fst64::mul_rn;
+using fst64::twice;
 
 // ---------------------------------------------------------------------------
 // k_prim3d: calculateRhoPT3D (src/secondary.hpp:109-151), computeVelocity3D
 // (src/velocity.hpp:68-83) over all cells; maxWaveSpeed (src/ceq3d.hpp:25-63)
 // and maxGradFunctor(var, nv+1) (src/ceq3d.hpp:82-93) over the interior.
+// Sums on the FP64 unit, the rest on the integer pipes; both about half busy, so
+// warps in flight matter: 5 blocks per SM (48 registers) 0.72 ms at 192^3 and 5
+// species, 4 blocks 0.77, 3 blocks 0.84 (operators throughout: 1.08 after the
+// integer division, 2.4 before it).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __restrict__ U,
+__global__ void __launch_bounds__(256, 5) k_prim3d(Geo g, Phys P, const double* __restrict__ U,
                                                 double* __restrict__ rho, double* __restrict__ pr,
                                                 double* __restrict__ vel, double* __restrict__ Y,
                                                 double* __restrict__ nrg, double* __restrict__ T,
@@ -44,21 +52,23 @@ __global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __r
                                                 const double* __restrict__ met) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long sv = g.sv;
-  double lS = -1.7976931348623157e308, lC = -1.7976931348623157e308;
+  const fst64::Fused k(P.ns);
+  unsigned long long kS = FST_KEY_LOWEST, kC = FST_KEY_LOWEST;
   if (c < sv) {
     double r = 0.0;
-    for (int s = 0; s < P.ns; ++s) r = r + U[c + sv * (4 + s)];
+    for (int s = 0; s < P.ns; ++s) r = k.add(r, U[c + sv * (4 + s)]);
     const fst64::Recip rr = fst64::recip_of(r);
     double Cp = 0, Cv = 0;
     for (int s = 0; s < P.ns; ++s) {
       double ys = div_by(U[c + sv * (4 + s)], rr);
-      Cp = Cp + ys * P.cp_s[s];
-      Cv = Cv + ys * P.cv_s[s];
+      Cp = k.add(Cp, mul_rn(ys, P.cp_s[s]));
+      Cv = k.add(Cv, mul_rn(ys, P.cv_s[s]));
       if (Y) Y[c + sv * s] = ys;
     }
     const double gam = div_rn(Cp, Cv);
     const double m0 = U[c], m1 = U[c + sv], m2 = U[c + 2 * sv], E = U[c + 3 * sv];
-    const double p = (gam - 1) * (E - div_by(0.5, rr) * (m0 * m0 + m1 * m1 + m2 * m2));
+    const double mm = k.add(k.add(mul_rn(m0, m0), mul_rn(m1, m1)), mul_rn(m2, m2));
+    const double p = mul_rn(k.sub(gam, 1.0), k.sub(E, mul_rn(div_by(0.5, rr), mm)));
     const double u = div_by(m0, rr), v = div_by(m1, rr), w = div_by(m2, rr);
     rho[c] = r;
     pr[c] = p;
@@ -69,124 +79,134 @@ __global__ void __launch_bounds__(256) k_prim3d(Geo g, Phys P, const double* __r
       for (int a = 0; a < 3; ++a) {
         const double* M = met + c + sv * a;
         vel[c + sv * a] =
-            div_by(M[0] * m0, rr) + div_by(M[3 * sv] * m1, rr) + div_by(M[6 * sv] * m2, rr);
+            k.add(k.add(div_by(mul_rn(M[0], m0), rr), div_by(mul_rn(M[3 * sv], m1), rr)),
+                  div_by(mul_rn(M[6 * sv], m2), rr));
       }
     } else {
       vel[c] = u;
       vel[c + sv] = v;
       vel[c + 2 * sv] = w;
     }
-    if (T) T[c] = div_rn(p, (Cp - Cv) * r);
+    if (T) T[c] = div_rn(p, mul_rn(k.sub(Cp, Cv), r));
     // specific internal energy of calculateRhoGrad::nrg (src/ceq3d.hpp:137-141)
-    if (nrg) nrg[c] = div_by(E, rr) - 0.5 * r * (u * u + v * v + w * w);
+    if (nrg) nrg[c] = k.sub(div_by(E, rr), mul_rn(half(r), k.add(k.add(mul_rn(u, u), mul_rn(v, v)),
+                                                                 mul_rn(w, w))));
     if (red) {
-      int i = (int)(c % g.sy), j = (int)((c / g.sy) % g.ngj), k = (int)(c / g.sz);
+      int i = (int)(c % g.sy), j = (int)((c / g.sy) % g.ngj), kk = (int)(c / g.sz);
       bool in = i >= g.ng && i < g.ngi - g.ng && j >= g.ng && j < g.ngj - g.ng &&
-                k >= g.ng && k < g.ngk - g.ng;
+                kk >= g.ng && kk < g.ngk - g.ng;
       if (in) {
-        double a = sqrt(div_by(gam * p, rr));
-        double s = a + div_by(sqrt(m0 * m0 + m1 * m1 + m2 * m2), rr);
-        if (s > lS) lS = s;
-        double ch = fabs(U[c + sv * (P.nv + 1)]);
-        if (ch > lC) lC = ch;
+        double a = sqrt(div_by(mul_rn(gam, p), rr));
+        double s = k.add(a, div_by(sqrt(mm), rr));
+        fst_key_max(kS, s);
+        fst_key_max(kC, fabs(U[c + sv * (P.nv + 1)]));
       }
     }
   }
-  if (red) {
-    lS = fst_warp_max(lS);
-    lC = fst_warp_max(lC);
-    if ((threadIdx.x & 31) == 0) {
-      atomicMax(&red[0], fst_key(lS));
-      atomicMax(&red[1], fst_key(lC));
+  if (red) fst_key_max_block<8>(red, kS, kC);
+}
+
+// ---------------------------------------------------------------------------
+// k_faces3d: the faces with normal F of the interior cells, the 9 velocity
+// gradients G[d][w] (derivative along d of velocity w) of each, then
+//  - the viscous stress components that the momenta take on that face
+//    (calculateStressTensor{x,y,z}3dv, src/viscosity.hpp:416-459, 499-541,
+//    581-624), S[(F*6 + w)*sv + cell], and the products of each with the face's
+//    mean velocity for the energy (applyViscousTerm*, :460-663), S[(F*6+3+w)*sv + cell]
+//  - C-equation face terms: calculateCeqFaces * calculateCeqGrads
+//    (src/ceq3d.hpp:226-332), MF[((F*3+d)*3+w)*sv + cell]
+// The reference evaluates each gradient twice (stress and C-equation) with
+// the same operations up to operand order of a commutative add, so the
+// values are identical and are computed once here.
+// One launch covers the three normals (blockIdx.x % 3): a block runs one of them.
+// Sums and the last products run on the FP64 unit, all else on the integer pipes
+// (fst_fp64.cuh), products and divisions as calls.  Measured at 192^3, 5 species,
+// per launch: 6.4 ms with all of it inlined (the warps wait for instructions),
+// 4.34 with calls, 3.74 at 7 blocks per SM instead of 5, 3.49 with 12 of a face's
+// products on the FP64 unit, which then is as busy as the integer one.
+// ---------------------------------------------------------------------------
+template <int F>
+__device__ __forceinline__ void face_terms3d(const Geo& g, const Phys& P, const fst64::Fused& k,
+                                             long long c, const double* __restrict__ U,
+                                             const double* __restrict__ rho,
+                                             const double* __restrict__ vel,
+                                             const double* __restrict__ Y,
+                                             const unsigned long long* __restrict__ red,
+                                             double* __restrict__ S, double* __restrict__ MF) {
+  constexpr int A = F == 0 ? 1 : 0, B = F == 2 ? 1 : 2;  // the tangential axes
+  const long long sv = g.sv;
+  const long long st[3] = {1, g.sy, g.sz};
+  const long long sf = st[F];  // outward normal step
+  double G[3][3], um[3];
+#pragma unroll
+  for (int w = 0; w < 3; ++w) {
+    const double* u = vel + sv * w;
+    const double u0 = u[c], u1 = u[c + sf];
+    G[F][w] = P.dd[F].call(k.sub(u1, u0));
+    um[w] = half(k.add(u1, u0));
+    auto tangential = [&](int d) {
+      const long long t = st[d];
+      return P.d4[d].call(k.sub(k.add(u[c + sf + t], u[c + t]), k.add(u[c + sf - t], u[c - t])));
+    };
+    G[A][w] = tangential(A);
+    G[B][w] = tangential(B);
+  }
+  if (P.visc) {
+    double mu = 0.0;
+    for (int s = 0; s < P.ns; ++s)
+      mu = k.add(mu, mul_call(half(k.add(Y[c + sf + sv * s], Y[c + sv * s])), P.mu_s[s]));
+    const double m23 = mul_call(2.0 / 3.0, mu);
+    double* Sf = S + (long long)F * 6 * sv + c;
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {
+      const double T = w == F ? mul_call(m23, k.sub(k.sub(twice(G[F][F]), G[A][A]), G[B][B]))
+                              : mul_call(mu, k.add(G[w][F], G[F][w]));
+      Sf[w * sv] = T;
+      Sf[(3 + w) * sv] = k.mul(um[w], T);
+    }
+  }
+  if (P.ceq) {
+    const double maxCh = fst_unkey(red[1]);
+    const double alpha = mul_call(div_rn(P.dxmag2, k.add(maxCh, 1.0e-6)), P.alpha);  // src/cart3d.cpp:285
+    const double* C = U + sv * P.nv;
+    auto mean = [&](const double* a) { return half(k.add(a[c], a[c + sf])); };
+    const double ar = mul_call(mul_call(alpha, mean(rho)), mean(C + sv));
+    const double cn[3] = {mean(C + 2 * sv), mean(C + 3 * sv), mean(C + 4 * sv)};
+    double cc[3];  // cn[F] cn[d]
+#pragma unroll
+    for (int d = 0; d < 3; ++d) cc[d] = mul_call(cn[F], cn[d]);
+    double cmag = 1.0e-6;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) cmag = k.add(cmag, d == F ? cc[F] : mul_call(cn[d], cn[d]));
+    const fst64::Recip rmag = fst64::recip_of(cmag);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double M = k.sub(F == d ? 1.0 : 0.0, fst64::div_call(cc[d], rmag.hi, rmag.lo, rmag.R));
+      const double base = mul_call(ar, M);
+      double* MFd = MF + (long long)((F * 3 + d) * 3) * sv + c;
+#pragma unroll
+      for (int w = 0; w < 3; ++w) MFd[w * sv] = k.mul(base, G[d][w]);
     }
   }
 }
 
-// ---------------------------------------------------------------------------
-// k_faces3d: per face index, the 27 face velocity gradients G[f][d][w]
-// (derivative along d of velocity w on face f), then
-//  - viscous stress on x/y/z faces: calculateStressTensor{x,y,z}3dv
-//    (src/viscosity.hpp:416-459, 499-541, 581-624), S[(f*6+comp)*sv + cell]
-//  - C-equation face terms: calculateCeqFaces * calculateCeqGrads
-//    (src/ceq3d.hpp:226-332), MF[((f*3+d)*3+w)*sv + cell]
-// The reference evaluates each gradient twice (stress and C-equation) with
-// the same operations up to operand order of a commutative add, so the
-// values are identical and are computed once here.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_faces3d(Geo g, Phys P, const double* __restrict__ U,
+__global__ void __launch_bounds__(128, 7) k_faces3d(Geo g, Phys P, const double* __restrict__ U,
                                                  const double* __restrict__ rho,
                                                  const double* __restrict__ vel,
                                                  const double* __restrict__ Y,
                                                  const unsigned long long* __restrict__ red,
                                                  double* __restrict__ S, double* __restrict__ MF) {
-  const int i = g.ng - 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = g.ng - 1 + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = g.ng - 1 + blockIdx.z;
-  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || k >= g.ngk - g.ng) return;
-  const long long c = fst_idx(g, i, j, k);
-  const long long sv = g.sv, sx = 1, sy = g.sy, sz = g.sz;
-  double alpha = 0.0;
-  if (P.ceq) {
-    const double maxCh = fst_unkey(red[1]);
-    alpha = div_rn(P.dxmag2, maxCh + 1.0e-6) * P.alpha;  // src/cart3d.cpp:285
-  }
-#pragma unroll
-  for (int f = 0; f < 3; ++f) {
-    const long long sf = f == 0 ? sx : f == 1 ? sy : sz;  // outward normal step
-    double G[3][3];  // G[d][w]
-#pragma unroll
-    for (int w = 0; w < 3; ++w) {
-      const double* u = vel + sv * w;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        if (d == f) {
-          const DivC dd = d == 0 ? P.ddx : d == 1 ? P.ddy : P.ddz;
-          G[d][w] = dd(u[c + sf] - u[c]);
-        } else {
-          const long long st = d == 0 ? sx : d == 1 ? sy : sz;
-          const DivC dd = d == 0 ? P.d4x : d == 1 ? P.d4y : P.d4z;
-          G[d][w] = dd((u[c + sf + st] + u[c + st]) - (u[c + sf - st] + u[c - st]));
-        }
-      }
-    }
-    if (P.visc) {
-      double mu = 0.0;
-      for (int s = 0; s < P.ns; ++s)
-        mu += ((Y[c + sf + sv * s] + Y[c + sv * s]) / 2.0) * P.mu_s[s];
-      const double dudx = G[0][0], dvdx = G[0][1], dwdx = G[0][2];
-      const double dudy = G[1][0], dvdy = G[1][1], dwdy = G[1][2];
-      const double dudz = G[2][0], dvdz = G[2][1], dwdz = G[2][2];
-      double* Sf = S + (long long)f * 6 * sv + c;
-      Sf[0 * sv] = (2.0 / 3.0) * mu * (2.0 * dudx - dvdy - dwdz);
-      Sf[1 * sv] = (2.0 / 3.0) * mu * (2.0 * dvdy - dudx - dwdz);
-      Sf[2 * sv] = (2.0 / 3.0) * mu * (2.0 * dwdz - dudx - dvdy);
-      Sf[3 * sv] = mu * (dudy + dvdx);
-      Sf[4 * sv] = mu * (dudz + dwdx);
-      Sf[5 * sv] = mu * (dvdz + dwdy);
-    }
-    if (P.ceq) {
-      const int nv = P.nv;
-      const double r = (rho[c] + rho[c + sf]) / 2.0;
-      const double chat = (U[c + sv * (nv + 1)] + U[c + sf + sv * (nv + 1)]) / 2.0;
-      double cn[3];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) cn[q] = (U[c + sv * (nv + 2 + q)] + U[c + sf + sv * (nv + 2 + q)]) / 2.0;
-      double cmag = 1.0e-6;
-      cmag += cn[0] * cn[0];
-      cmag += cn[1] * cn[1];
-      cmag += cn[2] * cn[2];
-const fst64::Recip rmag = fst64::recip_of(cmag);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const double dirac = f == d ? 1.0 : 0.0;
-        const double M = dirac - div_by(cn[f] * cn[d], rmag);
-        const double base = alpha * r * chat * M;
-        double* MFd = MF + (long long)((f * 3 + d) * 3) * sv + c;
-#pragma unroll
-        for (int w = 0; w < 3; ++w) MFd[w * sv] = base * G[d][w];
-      }
-    }
-  }
+  const int f = blockIdx.x % 3;
+  // faces c + 1/2 along f for c from the last ghost, interior cells across
+  const int i = g.ng - (f == 0) + blockIdx.x / 3 * blockDim.x + threadIdx.x;
+  const int j = g.ng - (f == 1) + blockIdx.y * blockDim.y + threadIdx.y;
+  const int kk = g.ng - (f == 2) + blockIdx.z;
+  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || kk >= g.ngk - g.ng) return;
+  const long long c = fst_idx(g, i, j, kk);
+  const fst64::Fused k(P.nv);
+  if (f == 0) face_terms3d<0>(g, P, k, c, U, rho, vel, Y, red, S, MF);
+  else if (f == 1) face_terms3d<1>(g, P, k, c, U, rho, vel, Y, red, S, MF);
+  else face_terms3d<2>(g, P, k, c, U, rho, vel, Y, red, S, MF);
 }
 
 // ---------------------------------------------------------------------------
@@ -197,8 +217,12 @@ const fst64::Recip rmag = fst64::recip_of(cmag);
 // computeBuoyancy3D (src/buoyancy.hpp:22-47), applyViscousTerm{x,y,z}3dv
 // (src/viscosity.hpp:460-663), calculateRhoGrad (src/ceq3d.hpp:95-187),
 // updateCeq (:189-224), applyCeq (:334-366), Loop1/Loop2 (src/rk.cpp:42-69).
+// The variables that share nothing run in different blocks (blockIdx.x % roles):
+// the momenta and energy, the species (advection only), the C variables; loops
+// over the directions stay rolled.  Both keep the code of a block small and give
+// a small grid three times the warps.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(128) k_cell3d(Geo g, Phys P, const double* __restrict__ U,
+__global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* __restrict__ U,
                                                 const double* __restrict__ rho,
                                                 const double* __restrict__ pr,
                                                 const double* __restrict__ vel,
@@ -209,143 +233,153 @@ __global__ void __launch_bounds__(128) k_cell3d(Geo g, Phys P, const double* __r
                                                 const unsigned long long* __restrict__ red,
                                                 const double* Uold, double* Unew, double coef,
                                                 double* __restrict__ Rout,
-                                                const double* __restrict__ met) {
-  const int i = g.ng + blockIdx.x * blockDim.x + threadIdx.x;
+                                                const double* __restrict__ met, int roles) {
+  const int role = blockIdx.x % roles;
+  const int i = g.ng + blockIdx.x / roles * blockDim.x + threadIdx.x;
   const int j = g.ng + blockIdx.y * blockDim.y + threadIdx.y;
-  const int k = g.ng + blockIdx.z;
-  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || k >= g.ngk - g.ng) return;
-  const long long c = fst_idx(g, i, j, k);
+  const int kk = g.ng + blockIdx.z;
+  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || kk >= g.ngk - g.ng) return;
+  const long long c = fst_idx(g, i, j, kk);
   const long long sv = g.sv, sx = 1, sy = g.sy, sz = g.sz;
   const int nv = P.nv;
+  const fst64::Fused k(nv);
 
   auto emit = [&](int v, double R) {
     if (Rout) Rout[c + sv * v] = R;
-    else Unew[c + sv * v] = Uold[c + sv * v] + coef * R;
+    else Unew[c + sv * v] = k.add(Uold[c + sv * v], mul_call(coef, R));
   };
+  // -((Fx - Fx-) + (Fy - Fy-) + (Fz - Fz-))
   auto divF = [&](int v) {
     const double* Fx = F + sv * v;
     const double* Fy = F + sv * (nv + v);
     const double* Fz = F + sv * (2 * nv + v);
-    return -((Fx[c] - Fx[c - sx]) + (Fy[c] - Fy[c - sy]) + (Fz[c] - Fz[c - sz]));
+    return -k.add(k.add(k.sub(Fx[c], Fx[c - sx]), k.sub(Fy[c], Fy[c - sy])),
+                  k.sub(Fz[c], Fz[c - sz]));
   };
+  // ((a- - 8 b-) + 8 b+) - a+ of the four neighbours along a direction
+  auto d4sum = [&](double am, double bm, double bp, double ap) {
+    return k.sub(k.add(k.sub(am, eight(bm)), eight(bp)), ap);
+  };
+  auto stride = [&](int f) { return f == 0 ? sx : f == 1 ? sy : sz; };
 
-  double R0 = divF(0), R1 = divF(1), R2 = divF(2), R3 = divF(3);
-  // species: only the advective term
-  for (int v = 4; v < nv; ++v) emit(v, divF(v));
-
-  if (met) {
-    // applyGenPressureGradient3D (src/presgrad.hpp:72-146): fourth-order
-    // differences of p * m(a, w) along each computational direction a
-    auto d4m = [&](long long st, int a, int w) {
-      const double* m = met + sv * (a + 3 * w);
-      return div_rn(pr[c - 2 * st] * m[c - 2 * st] - 8.0 * pr[c - st] * m[c - st] +
-                        8.0 * pr[c + st] * m[c + st] - pr[c + 2 * st] * m[c + 2 * st],
-                    12.0);
-    };
-    R0 = R0 - (d4m(sx, 0, 0) + d4m(sy, 1, 0) + d4m(sz, 2, 0));
-    R1 = R1 - (d4m(sx, 0, 1) + d4m(sy, 1, 1) + d4m(sz, 2, 1));
-    R2 = R2 - (d4m(sx, 0, 2) + d4m(sy, 1, 2) + d4m(sz, 2, 2));
-  } else {  // pressure gradient; the reference uses dz = cd(2) for the z term
-    const double dxp =
-        P.d12x(pr[c - 2 * sx] - 8.0 * pr[c - sx] + 8.0 * pr[c + sx] - pr[c + 2 * sx]);
-    const double dyp =
-        P.d12y(pr[c - 2 * sy] - 8.0 * pr[c - sy] + 8.0 * pr[c + sy] - pr[c + 2 * sy]);
-    const double dzp =
-        P.d12pz(pr[c - 2 * sz] - 8.0 * pr[c - sz] + 8.0 * pr[c + sz] - pr[c + 2 * sz]);
-    R0 = R0 - dxp;
-    R1 = R1 - dyp;
-    R2 = R2 - dzp;
+  if (role == 1) {  // species: only the advective term
+#pragma unroll 1
+    for (int v = 4; v < nv; ++v) emit(v, divF(v));
+    // C-equation variables carried without a right-hand side (the generalized
+    // module evolves none): U + coef*0, as the reference's zero dvar gives
+    if (!P.ceq)
+      for (int v = nv; v < g.nvt; ++v) emit(v, 0.0);
+    return;
   }
-  if (P.buoyancy) {
-    const double vb = div_rn(U[c + sv], rho[c]);
-    const double rhop = rho[c] - P.rho_ref;
-    const double f = -P.g * rhop;
-    R1 += f;
-    R3 += vb * f;
-  }
-  if (P.visc) {
-    // stress components feeding (x-mom, y-mom, z-mom) on each face set
-    const int comp[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
-#pragma unroll
+  if (role == 2) {  // C variables: calculateRhoGrad, updateCeq
+    double gr[3], ge[3], divu = 0.0;
+#pragma unroll 1
     for (int f = 0; f < 3; ++f) {
-      const long long st = f == 0 ? sx : f == 1 ? sy : sz;
-      const DivC dd = f == 0 ? P.ddx : f == 1 ? P.ddy : P.ddz;
-      const double* Sf = S + (long long)f * 6 * sv;
-      const double* u0 = vel;
-      const double* u1 = vel + sv;
-      const double* u2 = vel + 2 * sv;
-      const double ur = (u0[c + st] + u0[c]) / 2.0, ul = (u0[c - st] + u0[c]) / 2.0;
-      const double vr = (u1[c + st] + u1[c]) / 2.0, vl = (u1[c - st] + u1[c]) / 2.0;
-      const double wr = (u2[c + st] + u2[c]) / 2.0, wl = (u2[c - st] + u2[c]) / 2.0;
-      const double s0 = Sf[comp[f][0] * sv + c], s0m = Sf[comp[f][0] * sv + c - st];
-      const double s1 = Sf[comp[f][1] * sv + c], s1m = Sf[comp[f][1] * sv + c - st];
-      const double s2 = Sf[comp[f][2] * sv + c], s2m = Sf[comp[f][2] * sv + c - st];
-      const double a = dd(s0 - s0m);
-      const double b = dd(s1 - s1m);
-      const double cc = dd(s2 - s2m);
-      const double d = dd(ur * s0 - ul * s0m) + dd(vr * s1 - vl * s1m) + dd(wr * s2 - wl * s2m);
-      R0 += a;
-      R1 += b;
-      R2 += cc;
-      R3 += d;
+      const long long s = stride(f);
+      const DivC& d12 = P.d12[f];
+      auto d4 = [&](const double* a) {
+        return d12.call(d4sum(a[c - 2 * s], a[c - s], a[c + s], a[c + 2 * s]));
+      };
+      const double r = d4(rho), e = d4(nrg), u = d4(vel + sv * f);
+      divu = f == 0 ? u : k.add(divu, u);
+      if (f == 0) { gr[0] = r; ge[0] = e; }
+      else if (f == 1) { gr[1] = r; ge[1] = e; }
+      else { gr[2] = r; ge[2] = e; }
     }
-  }
-  if (P.ceq) {
-    // calculateRhoGrad
-    auto d4 = [&](const double* a, long long st, const DivC& d12) {
-      return d12(a[c - 2 * st] - 8.0 * a[c - st] + 8.0 * a[c + st] - a[c + 2 * st]);
-    };
-    const double dxr = d4(rho, sx, P.d12x), dyr = d4(rho, sy, P.d12y), dzr = d4(rho, sz, P.d12z);
-    const double dxe = d4(nrg, sx, P.d12x), dye = d4(nrg, sy, P.d12y), dze = d4(nrg, sz, P.d12z);
-    const double dxu = d4(vel, sx, P.d12x), dyv = d4(vel + sv, sy, P.d12y),
-                 dzw = d4(vel + 2 * sv, sz, P.d12z);
-    const double n1 = dxr, n2 = dyr, n3 = dzr;
-    const double rgrad = sqrt(dxr * dxr + dyr * dyr + dzr * dzr);
-    const double divu = dxu + dyv + dzw;
-    const double dnednr = (n1 * dxe + n2 * dye + n3 * dze) * (n1 * dxr + n2 * dyr + n3 * dzr);
-    const int ind = dnednr < 0.0 ? 1 : 0;
-    double G[5];
-    G[0] = divu < 0 ? (1 - ind) * rgrad : 0.0;
-    G[1] = ind * rgrad;
-    G[2] = dxr;
-    G[3] = dyr;
-    G[4] = dzr;
-    // updateCeq
+    const double g2 = k.add(k.add(mul_call(gr[0], gr[0]), mul_call(gr[1], gr[1])), mul_call(gr[2], gr[2]));
+    const double rgrad = sqrt(g2);
+    const double dnednr = mul_call(
+        k.add(k.add(mul_call(gr[0], ge[0]), mul_call(gr[1], ge[1])), mul_call(gr[2], ge[2])), g2);
+    const bool ind = dnednr < 0.0;
     const double maxS = fst_unkey(red[0]);
     const double src = div_rn(maxS, P.eps * P.dxmag);
     const double dif = P.kap * maxS * P.dxmag;
-#pragma unroll
+#pragma unroll 1
     for (int n = 0; n < 5; ++n) {
+      // (1 - ind) rgrad, ind rgrad of the reference: the factors are 0 or 1
+      double Gn;
+      if (n == 0) Gn = divu < 0 ? mul_call(ind ? 0.0 : 1.0, rgrad) : 0.0;
+      else if (n == 1) Gn = mul_call(ind ? 1.0 : 0.0, rgrad);
+      else Gn = n == 2 ? gr[0] : n == 3 ? gr[1] : gr[2];
       const double* Cn = U + sv * (nv + n);
-      const double cc = Cn[c];
-      const double lap = P.ddx(Cn[c - sx] - 2 * cc + Cn[c + sx]) +
-                         P.ddy(Cn[c - sy] - 2 * cc + Cn[c + sy]) +
-                         P.ddz(Cn[c - sz] - 2 * cc + Cn[c + sz]);
-      emit(nv + n, src * (G[n] - cc) + dif * lap);
+      const double cc = Cn[c], c2 = twice(cc);
+      const double lx = P.dd[0].call(k.add(k.sub(Cn[c - sx], c2), Cn[c + sx]));
+      const double ly = P.dd[1].call(k.add(k.sub(Cn[c - sy], c2), Cn[c + sy]));
+      const double lz = P.dd[2].call(k.add(k.sub(Cn[c - sz], c2), Cn[c + sz]));
+      const double lap = k.add(k.add(lx, ly), lz);
+      emit(nv + n, k.add(mul_call(src, k.sub(Gn, cc)), mul_call(dif, lap)));
     }
-    // applyCeq
-    double diffu[3] = {0.0, 0.0, 0.0};
-#pragma unroll
+    return;
+  }
+
+  double R0 = divF(0), R1 = divF(1), R2 = divF(2), R3 = divF(3);
+  if (met) {
+    // applyGenPressureGradient3D (src/presgrad.hpp:72-146): fourth-order
+    // differences of p * m(a, w) along each computational direction a
+#pragma unroll 1
     for (int w = 0; w < 3; ++w) {
+      auto d4m = [&](long long s, int a) {
+        const double* m = met + sv * (a + 3 * w);
+        // 8.0 * p * m: the product with 8 first, exact
+        return div_rn(k.sub(k.add(k.sub(mul_call(pr[c - 2 * s], m[c - 2 * s]),
+                                        mul_call(eight(pr[c - s]), m[c - s])),
+                                  mul_call(eight(pr[c + s]), m[c + s])),
+                            mul_call(pr[c + 2 * s], m[c + 2 * s])),
+                      12.0);
+      };
+      const double d = k.add(k.add(d4m(sx, 0), d4m(sy, 1)), d4m(sz, 2));
+      if (w == 0) R0 = k.sub(R0, d);
+      else if (w == 1) R1 = k.sub(R1, d);
+      else R2 = k.sub(R2, d);
+    }
+  } else {  // pressure gradient; the reference uses dz = cd(2) for the z term
+#pragma unroll 1
+    for (int f = 0; f < 3; ++f) {
+      const long long s = stride(f);
+      const DivC& d12 = f == 2 ? P.d12pz : P.d12[f];
+      const double d = d12.call(d4sum(pr[c - 2 * s], pr[c - s], pr[c + s], pr[c + 2 * s]));
+      if (f == 0) R0 = k.sub(R0, d);
+      else if (f == 1) R1 = k.sub(R1, d);
+      else R2 = k.sub(R2, d);
+    }
+  }
+  if (P.buoyancy) {
+    const double vb = div_rn(U[c + sv], rho[c]);
+    const double f = mul_call(-P.g, k.sub(rho[c], P.rho_ref));
+    R1 = k.add(R1, f);
+    R3 = k.add(R3, mul_call(vb, f));
+  }
+  if (P.visc) {
+#pragma unroll 1
+    for (int f = 0; f < 3; ++f) {
+      const long long s = stride(f);
+      const DivC& dd = P.dd[f];
+      const double* Sf = S + (long long)f * 6 * sv + c;
+      auto diff = [&](int q) { return dd.call(k.sub(Sf[q * sv], Sf[q * sv - s])); };
+      R0 = k.add(R0, diff(0));
+      R1 = k.add(R1, diff(1));
+      R2 = k.add(R2, diff(2));
+      R3 = k.add(R3, k.add(k.add(diff(3), diff(4)), diff(5)));
+    }
+  }
+  if (P.ceq) {  // applyCeq
+    double diffu[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int f = 0; f < 3; ++f) {
+      const long long s = stride(f);
+      const DivC& dd = P.dd[f];
+#pragma unroll 1
+      for (int d = 0; d < 3; ++d) {
+        const double* m = MF + (long long)((f * 3 + d) * 3) * sv + c;
 #pragma unroll
-      for (int f = 0; f < 3; ++f) {
-        const long long st = f == 0 ? sx : f == 1 ? sy : sz;
-        const DivC dd = f == 0 ? P.ddx : f == 1 ? P.ddy : P.ddz;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double* m = MF + (long long)((f * 3 + d) * 3 + w) * sv;
-          diffu[w] += dd(m[c] - m[c - st]);
-        }
+        for (int w = 0; w < 3; ++w)
+          diffu[w] = k.add(diffu[w], dd.call(k.sub(m[w * sv], m[w * sv - s])));
       }
     }
-    R0 += diffu[0];
-    R1 += diffu[1];
-    R2 += diffu[2];
+    R0 = k.add(R0, diffu[0]);
+    R1 = k.add(R1, diffu[1]);
+    R2 = k.add(R2, diffu[2]);
   }
-  // C-equation variables carried without a right-hand side (the generalized
-  // module evolves none): U + coef*0, as the reference's zero dvar gives
-  if (!P.ceq)
-    for (int v = nv; v < g.nvt; ++v) emit(v, 0.0);
   emit(0, R0);
   emit(1, R1);
   emit(2, R2);
@@ -390,12 +424,13 @@ int fst_plain3d_stage(const Geo& g, const Phys& P, const Plain3DBufs& b, const d
   FST_LAUNCH(prof, "flux3d", st, n, fstflux::launch<true>(g, P, 3, Uin, b.pr, b.vel, b.F, st));
   if (P.visc || P.ceq) {
     FST_LAUNCH(prof, "faces3d", st, n,
-               k_faces3d<<<gf, bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.Y, b.red, b.S, b.MF));
+               k_faces3d<<<dim3(3 * gf.x, gf.y, gf.z), bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.Y, b.red, b.S, b.MF));
   }
-  const dim3 gc(cdiv(g.nci, 32), cdiv(g.ncj, 4), g.nck);
+  const int roles = P.ceq ? 3 : 2;
+  const dim3 gc(cdiv(g.nci, 32) * roles, cdiv(g.ncj, 4), g.nck);
   FST_LAUNCH(prof, "cell3d", st, n,
              k_cell3d<<<gc, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.MF,
-                                         b.red, Uold, Unew, coef, Rout, b.met));
+                                         b.red, Uold, Unew, coef, Rout, b.met, roles));
   if (ghosts && !Rout)
     FST_LAUNCH(prof, "ghost3d", st, n,
                k_ghost3d<<<cdiv(g.sv, 256), 256, 0, st>>>(g, Uold, Unew, coef));

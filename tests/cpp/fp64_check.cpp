@@ -47,7 +47,7 @@ extern "C" long long fp64_check(long long n, uint64_t seed) {
   const double edge[] = {0.0, -0.0, 1.0, -1.0, INFINITY, -INFINITY, NAN, 4.9e-324, 2.2250738585072014e-308,
                          1.7976931348623157e308, 1e-300, 1e300, 3.0, 0.1};
   for (double a : edge)
-    for (double b : edge) bad += !same(a / b, div_rn(a, b));
+    for (double b : edge) bad += !same(a / b, div_rn(a, b)) + !same(a * b, mul_rn(a, b));
   for (double a : edge)
     for (int k = -900; k <= 900; k += 7) bad += !same(a * std::ldexp(1.0, k), scale2(a, k, std::ldexp(1.0, k)));
   for (long long q = 0; q < n; ++q) {
@@ -60,6 +60,8 @@ extern "C" long long fp64_check(long long n, uint64_t seed) {
     }
     bad += !same(a / b, div_rn(a, b));
     bad += !same(a / b, div_by(a, recip_of(b)));
+    bad += !same(a * b, mul_rn(a, b));
+    bad += !same(a * 0.5, half(a)) + !same(a * 2.0, twice(a)) + !same(a * 8.0, eight(a));
     const int k = (int)(r() % 2000) - 1000;
     bad += !same(a * std::ldexp(1.0, k), scale2(a, k, std::ldexp(1.0, k)));
     // the products' ranges: a normal or zero, the result normal
