@@ -152,7 +152,8 @@ struct Plan {
 // first form the face velocities, then each warp marches one variable after
 // another along the 32 lines.  Lanes run along the first transverse axis, so loads
 // and stores of the y and z directions are coalesced; along x a warp walks 32 rows
-// side by side and reuses each memory line it fetched for 16 steps.  More warps in
+// side by side and reuses each memory line it fetched for 16 steps.  gridDim.y
+// blocks share the variables.  More warps in
 // flight than the 16 to 20 of this split gain nothing (18 to 28: 2 %).
 // Face values go to F[(dir*nv + v)*sv + cell] for the faces of interior cells.
 constexpr int WMAX = 5;  // warps per block, at most
@@ -194,7 +195,7 @@ __global__ void __launch_bounds__(32 * WMAX, 4)
   __syncthreads();
 
   const double* pq = pr + line;
-  for (int v = warp; v < nv; v += nwarp) {
+  for (int v = warp + nwarp * blockIdx.y; v < nv; v += nwarp * gridDim.y) {
     const double* q = U + sv * v + line;
     double* Fd = F + sv * ((long long)dir * nv + v) + line;
     // stencil value of a cell: var + (v==energy)*p.  For the others that is
@@ -296,12 +297,13 @@ inline Plan make_plan(const Geo& g, const Phys& P) {
     D.dd = dd[d];
     chunks += (long long)((D.lines + 31) / 32) * (D.n + 1);
   }
-  // faces per segment: the whole launch should have about 8 warps per
-  // sub-partition or more (a segment of 4 already spends a third of its work on
-  // the cell terms of its first faces)
-  const long long want = 8LL * 4 * 152;
+  // faces per segment: as many as leave the launch 16 warps per sub-partition, 2 at
+  // least (a segment starts with the work of about three faces).  Measured against
+  // 8 warps and 4 faces at least, per launch: 24x20x16 33 -> 21 us, 64x48 18 -> 13,
+  // 64^3 487 -> 428 (with the split below), 800x700 491 -> 407; 32 warps: 449, 406.
+  const long long want = 16LL * 4 * 152;
   int len = LSEG;
-  while (len > 4 && chunks * g.nv / len < want) len >>= 1;
+  while (len > 2 && chunks * g.nv / len < want) len >>= 1;
   int first = 0;
   for (int d = 0; d < g.ndim; ++d) {
     Dir& D = p.d[d];
@@ -322,7 +324,12 @@ inline void launch(const Geo& g, const Phys& P, int ve, const double* U, const d
   int w = WMAX;
   for (int q = WMAX - 1; q >= 3; --q)
     if ((g.nv + q - 1) / q * q < (g.nv + w - 1) / w * w) w = q;
-  k_weno_flux<F32><<<p.blocks, 32 * w, 0, st>>>(p, g.sv, g.nv, ve, U, pr, vel, F);
+  // The rounds of a block's warps over the variables become blocks of their own
+  // below 16 waves of blocks, where the last wave counts (64^3 487 -> 445 us); above,
+  // forming the face velocities once per round costs more (192^3 10.43 -> 10.85 ms).
+  const int rounds = (g.nv + w - 1) / w;
+  const int split = p.blocks <= 16 * 4 * 152 ? rounds : 1;
+  k_weno_flux<F32><<<dim3(p.blocks, split), 32 * w, 0, st>>>(p, g.sv, g.nv, ve, U, pr, vel, F);
 }
 
 }  // namespace fstflux
