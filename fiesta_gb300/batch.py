@@ -6,7 +6,7 @@ import math
 import numpy as np
 
 from . import abi
-from .solver import FstError, initial_conditions, lib
+from .solver import FstError, host_array, initial_conditions, lib
 
 
 class BatchInfo(C.Structure):
@@ -75,7 +75,7 @@ class Batch:
                                              U.size), "set_state")
 
     def get_state(self, c):
-        U = np.zeros(abi.dims(self.cfgs[c]), dtype=np.float64, order="F")
+        U = host_array(abi.dims(self.cfgs[c]))
         self._check(_L().fst_batch_get_state(self._b, c, U.ctypes.data_as(C.POINTER(C.c_double)),
                                              U.size), "get_state")
         return U
