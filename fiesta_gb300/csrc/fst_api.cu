@@ -63,6 +63,7 @@ struct fst_ctx {
   // fst_rk_step_get_state: the side stream of the overlapped download
   MixedDownload dl{};
   int* dflag = nullptr;
+  fstbc::GhostRule rule{};  // how the ghost cells are filled
   bool gen = false;       // FST_GRID_GENERALIZED
   bool grid_set = false;  // fst_set_grid has computed the metrics
   Prof prof;
@@ -348,8 +349,8 @@ int stage(fst_ctx* c, const double* Uin, const double* Uold, double* Unew, doubl
   return check_launch(c, "stage kernels");
 }
 
-int bcs(fst_ctx* c, double* U) {
-  c->stats.kernel_launches += fst_launch_bcs(c->g, c->cf, U, c->stream, &c->prof);
+int bcs(fst_ctx* c, double* U, double* U2 = nullptr) {
+  c->stats.kernel_launches += fst_launch_bcs(c->g, c->cf, U, c->stream, &c->prof, U2);
   return check_launch(c, "boundary kernels");
 }
 
@@ -420,6 +421,7 @@ int fst_create(const fst_config* cfg, fst_ctx** out) {
   g.sz = (long long)g.ngi * g.ngj;
   g.sv = g.sz * g.ngk;
   setup_phys(*cfg, g, c->P);
+  c->rule = fstbc::ghost_rule(g, *cfg);
 
   const size_t cells = (size_t)g.sv;
   const size_t need = cells * sizeof(double) * (2 * (size_t)g.nvt + work_doubles_per_cell(*cfg, g));
@@ -475,7 +477,7 @@ int fst_create(const fst_config* cfg, fst_ctx** out) {
     rc = fst_mixed_alloc(*cfg, g, c->bm, [&](void** p, size_t bytes) { return alloc(c, p, bytes); },
                          &why);
     if (rc && !why.empty()) fail(c, rc, why);
-    c->bm.rule = fstbc::ghost_rule(g, *cfg);
+    c->bm.rule = c->rule;
   }
   // zero state like a fresh Kokkos View; zero work arrays so that entries
   // outside each kernel's range read as the reference's zero-initialised ones
@@ -678,12 +680,14 @@ int one_step(fst_ctx* c) {
     return c->bm.fill ? FST_OK : bcs(c, U);
   };
   // Stage 1 copies the ghosts into its buffer (U + (0.5 dt) 0, src/rk.cpp:42-50)
-  // where they are read: always in 2D and on generalized grids, in 3D only where
-  // a fill with fewer cells than ghost layers reads ghosts.
-  const bool keep = !cart3 || g.nci < g.ng || g.ncj < g.ng || g.nck < g.ng;
+  // where they are read and nothing else writes them: on generalized grids, in 3D
+  // where a fill with fewer cells than ghost layers reads ghosts, and in 2D unless
+  // the one-launch fill, whose ghosts both stages read, has written both buffers.
+  const bool both = g.ndim == 2 && !c->gen && c->rule.direct && fst_shell_count(g) < (1LL << 31);
+  const bool keep = cart3 ? g.nci < g.ng || g.ncj < g.ng || g.nck < g.ng : !both;
   // gen2d / gen3d apply no boundary conditions (src/gen2d.cpp:132-134,
   // src/gen3d.cpp:109, 338-370)
-  if (g.ndim == 2 && !c->gen) rc = bcs(c, c->Ua);  // cart2d_func::preStep
+  if (g.ndim == 2 && !c->gen) rc = bcs(c, c->Ua, c->Ub);  // cart2d_func::preStep
   if (cart3) rc = ghosts(c->Ua);
   c->bm.stage = 1;
   MixedDownload* dl = c->bm.dl;

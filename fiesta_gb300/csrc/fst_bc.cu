@@ -9,9 +9,9 @@
 // are separate launches because later axes read ghosts written by earlier
 // ones; the two faces of an axis share a launch when they touch disjoint
 // cells.  One thread owns one ghost line and runs the reference's per-line
-// loop in the reference's order.  Where the sequence amounts to one copy per ghost
-// cell (no hydrostatic face, at least ng cells per axis) a single launch makes
-// those copies instead, with the same values.
+// loop in the reference's order.  Where every ghost cell follows from interior
+// cells alone (fstbc::ghost_rule) a single launch fills them instead, with the same
+// values.
 //
 // Built with --fmad=false: the hydrostatic energy extrapolation must round
 // exactly as the reference does.
@@ -45,25 +45,36 @@ __global__ void k_face(Geo g, double* __restrict__ U, int axis, int side, int ty
 }
 
 // Every ghost cell in one launch (fstbc::GhostRule): a thread copies VC variables
-// of one ghost cell, its loads in flight together.
+// of one ghost cell, its loads in flight together; to U2 as well when given (the
+// 2D stage-1 buffer, whose ghosts are those of the state).
 constexpr int VC = 5;
 __global__ void __launch_bounds__(128) k_ghosts(Geo g, fstbc::GhostRule r, double* __restrict__ U,
-                                                int nshell) {
+                                                double* __restrict__ U2, int nshell) {
   const int t = blockIdx.x * 128 + threadIdx.x;
   if (t >= nshell) return;
   int i, j, k;
   fst_shell_cell(g, t, i, j, k);
   const long long dst = fst_idx(g, i, j, k);
-  const unsigned flip = fstbc::ghost_source(g, r, i, j, k);
-  const long long src = fst_idx(g, i, j, k);
+  const fstbc::GhostSource s = fstbc::ghost_source(g, r, i, j, k);
   const int v0 = blockIdx.y * VC;
   double x[VC];
 #pragma unroll
   for (int q = 0; q < VC; ++q)
-    if (v0 + q < g.nvt) x[q] = U[src + g.sv * (v0 + q)];
+    if (v0 + q < g.nvt) x[q] = U[s.src + g.sv * (v0 + q)];
+  if (s.layer >= 0 && v0 <= g.ndim && g.ndim < v0 + VC) {
+    const double e = fstbc::ghost_energy(g, U, s);
+#pragma unroll
+    for (int q = 0; q < VC; ++q)
+      if (v0 + q == g.ndim) x[q] = e;
+  }
 #pragma unroll
   for (int q = 0; q < VC; ++q)
-    if (v0 + q < g.nvt) U[dst + g.sv * (v0 + q)] = fstbc::ghost_value(x[q], flip, v0 + q);
+    if (v0 + q < g.nvt) {
+      const bool e = s.layer >= 0 && v0 + q == g.ndim;
+      const double y = e ? x[q] : fstbc::ghost_value(x[q], s.flip, v0 + q);
+      U[dst + g.sv * (v0 + q)] = y;
+      if (U2) U2[dst + g.sv * (v0 + q)] = y;
+    }
 }
 
 inline unsigned nblk(long long n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -81,16 +92,18 @@ void fst_fill_keys(unsigned long long* p, int n, unsigned long long v, cudaStrea
   if (n > 0) k_fill_keys<<<nblk(n, 64), 64, 0, st>>>(p, n, v);
 }
 
-// Host launcher: the whole applyBCs sequence on `stream`.  Returns the number
-// of kernels launched.
-int fst_launch_bcs(const Geo& g, const fst_config& cf, double* U, cudaStream_t stream, Prof* prof) {
+// Host launcher: the whole applyBCs sequence on `stream`.  U2, where the rule is
+// direct: a second state that gets the same ghost cells (else it is left alone).
+// Returns the number of kernels launched.
+int fst_launch_bcs(const Geo& g, const fst_config& cf, double* U, cudaStream_t stream, Prof* prof,
+                   double* U2) {
   int launches = 0;
   const int B = 128;
   const fstbc::GhostRule rule = fstbc::ghost_rule(g, cf);
   const long long shell = fst_shell_count(g);
   if (rule.direct && shell < (1LL << 31)) {
     FST_LAUNCH(prof, "bc_ghosts", stream, launches,
-               k_ghosts<<<dim3(nblk(shell, B), nblk(g.nvt, VC)), B, 0, stream>>>(g, rule, U,
+               k_ghosts<<<dim3(nblk(shell, B), nblk(g.nvt, VC)), B, 0, stream>>>(g, rule, U, U2,
                                                                                  (int)shell));
     return launches;
   }

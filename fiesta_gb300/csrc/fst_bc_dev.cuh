@@ -103,11 +103,15 @@ __device__ __forceinline__ void face_line(const Geo& g, double* __restrict__ U, 
 }
 
 // ---------------------------------------------------------------------------
-// Every ghost cell at once.  With at least ng cells on every axis and no
-// hydrostatic face, the sequence of fills leaves in a ghost cell the value of one
-// interior cell, found axis by axis (each fill runs over the full transverse
-// extent, so a later one copies what an earlier one wrote), with the signs of the
-// axes' reflections multiplied.
+// Every ghost cell at once.  With at least ng cells on every axis the sequence of
+// fills leaves in a ghost cell the value of one interior cell, found axis by axis
+// (each fill runs over the full transverse extent, so a later one copies what an
+// earlier one wrote), with the signs of the axes' reflections multiplied.  The
+// energy beyond a hydrostatic face is the exception: an extrapolation along the
+// face's normal.  On the axis filled last (the last non-periodic one) it reads, on
+// its line, copies of interior cells only, so a ghost cell's energy still follows
+// from up to three interior cells.  A hydrostatic face on an axis filled earlier
+// takes the fills one after another.
 // ---------------------------------------------------------------------------
 struct GhostRule {
   int direct;       // 0: the fills have to run one after another
@@ -120,43 +124,84 @@ inline GhostRule ghost_rule(const Geo& g, const fst_config& cf) {
   const int n[3] = {g.nci, g.ncj, g.nck};
   const int per[3] = {cf.xper != 0, cf.yper != 0, cf.zper != 0};
   const int t[3][2] = {{cf.bc_xmin, cf.bc_xmax}, {cf.bc_ymin, cf.bc_ymax}, {cf.bc_zmin, cf.bc_zmax}};
-  r.direct = 1;
+  int last = -1;
+  for (int a = 0; a < g.ndim; ++a)
+    if (!per[a]) last = a;
+  r.direct = g.ng == 3;
   for (int a = 0; a < g.ndim; ++a) {
     r.per[a] = per[a];
     for (int s = 0; s < 2; ++s) {
       r.type[a][s] = t[a][s];
-      if (!per[a] && t[a][s] == FST_BC_HYDROSTATIC) r.direct = 0;
+      if (!per[a] && a != last && t[a][s] == FST_BC_HYDROSTATIC) r.direct = 0;
     }
     if (n[a] < g.ng) r.direct = 0;
   }
   return r;
 }
 
-// The interior cell behind ghost cell (i, j, k), in place, and the variables
-// 0..2 whose sign it takes flipped (bit v).
-__device__ __forceinline__ unsigned ghost_source(const Geo& g, const GhostRule& r, int& i, int& j,
-                                                 int& k) {
-  unsigned flip = 0;
-  auto axis = [&](int a, int& x, int n) {
+// Where a ghost cell's values come from: the interior cell `src`, the variables
+// 0..2 whose sign is flipped (bit v), and for a ghost cell beyond a hydrostatic
+// face its layer (0 nearest, else -1) and the stride from a cell of its line to the
+// next one inward.
+struct GhostSource {
+  long long src, inward;
+  unsigned flip;
+  int layer;
+};
+__device__ __forceinline__ GhostSource ghost_source(const Geo& g, const GhostRule& r, int i, int j,
+                                                    int k) {
+  GhostSource q{0, 0, 0u, -1};
+  auto axis = [&](int a, int& x, int n, long long stride) {
     const int side = x < g.ng ? 0 : x >= g.ng + n ? 1 : -1;
     if (side < 0) return;
     if (r.per[a]) {
       x += side ? -n : n;
       return;
     }
-    x = side ? 2 * (g.ng + n) - 1 - x : 2 * g.ng - 1 - x;
+    const int layer = side ? x - (g.ng + n) : g.ng - 1 - x;
+    x = side ? g.ng + n - 1 - layer : g.ng + layer;
     const int t = r.type[a][side];
-    flip ^= t == FST_BC_NOSLIP ? 7u : t == FST_BC_REFLECTIVE ? 1u << a : 0u;
+    q.flip ^= t == FST_BC_NOSLIP ? 7u : t == FST_BC_OUTFLOW ? 0u : 1u << a;
+    if (t == FST_BC_HYDROSTATIC) {
+      q.layer = layer;
+      q.inward = side ? -stride : stride;
+    }
   };
-  axis(0, i, g.nci);
-  axis(1, j, g.ncj);
-  if (g.ndim == 3) axis(2, k, g.nck);
-  return flip;
+  axis(0, i, g.nci, 1);
+  axis(1, j, g.ncj, g.sy);
+  if (g.ndim == 3) axis(2, k, g.nck, g.sz);
+  q.src = fst_idx(g, i, j, k);
+  return q;
 }
 // x, its sign flipped when bit v of flip is set (what multiplying by -1 gives)
 __device__ __forceinline__ double ghost_value(double x, unsigned flip, int v) {
   const unsigned long long b = fst64::bits_of(x);
   return fst64::of_bits(v < 3 && ((flip >> v) & 1) ? b ^ 0x8000000000000000ull : b);
+}
+// The energy of a ghost cell beyond a hydrostatic face (q.layer >= 0): the linear
+// extrapolation of face_line above, layer after layer outward; the ghost layers'
+// kinetic energies are those of the interior layers they mirror.
+__device__ __forceinline__ double ghost_energy(const Geo& g, const double* U, const GhostSource& q) {
+  const long long c0 = q.src - q.inward * q.layer;  // the line's first interior cell
+  const int edx = g.ndim, rdx = g.ndim + 1;
+  auto kinetic = [&](int n) {
+    const long long c = c0 + q.inward * n;
+    double ke = 0;
+    for (int d = 0; d < g.ndim; ++d) {
+      const double u = U[c + g.sv * d];
+      ke += 0.5 * (u * u);
+    }
+    return ke / U[c + g.sv * rdx];
+  };
+  const double ke0 = kinetic(0), ke1 = kinetic(1);
+  // (in 2D a no-slip face on the other axis has flipped the energy)
+  const double E0 = ghost_value(U[c0 + g.sv * edx], q.flip, edx);
+  const double E1 = ghost_value(U[c0 + q.inward + g.sv * edx], q.flip, edx);
+  const double g0 = 2 * (E0 - ke0) - (E1 - ke1) + ke0;
+  if (q.layer == 0) return g0;
+  const double g1 = 2 * (g0 - ke0) - (E0 - ke0) + ke1;
+  if (q.layer == 1) return g1;
+  return 2 * (g1 - ke1) - (g0 - ke0) + kinetic(2);
 }
 
 }  // namespace fstbc

@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(128) k_mfill3_shell(Geo g, Geo gq, Phys P, fst
   const long long sv = g.sv;
   const long long dst = (long long)i + g.sy * j + g.sz * k;
   const long long q = (long long)i + gq.sy * j + gq.sz * k;
-  const unsigned flip = fstbc::ghost_source(g, rule, i, j, k);
-  const long long src = (long long)i + g.sy * j + g.sz * k;
+  const fstbc::GhostSource gs = fstbc::ghost_source(g, rule, i, j, k);
+  const long long src = gs.src;
   const bool ceq = g.nvt > g.nv;
   double us[NS], um[4], uc[5];
 #pragma unroll
@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(128) k_mfill3_shell(Geo g, Geo gq, Phys P, fst
     for (int n = 0; n < 5; ++n) uc[n] = U[src + sv * (g.nv + n)];
   }
 #pragma unroll
-  for (int d = 0; d < 3; ++d) um[d] = fstbc::ghost_value(um[d], flip, d);
+  for (int d = 0; d < 3; ++d) um[d] = fstbc::ghost_value(um[d], gs.flip, d);
+  if (gs.layer >= 0) um[3] = fstbc::ghost_energy(g, U, gs);
   if (store) {
 #pragma unroll
     for (int d = 0; d < 4; ++d) U[dst + sv * d] = um[d];
