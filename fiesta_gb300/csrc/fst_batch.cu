@@ -3,8 +3,11 @@
 //
 // Per RK stage the ensemble is advanced by a fixed set of launches that
 // cover every case at once, instead of one set per case:
-//   k_bface / k_bperiodic  ghost fills, one launch per fill step, grid.y = case
-//   k_binit                reset the per-case C-equation maxima
+//   k_bfill                ghost rows and columns of both stage buffers, grid.y = case
+//                          (k_bperiodic / k_bface, one launch per fill step, and
+//                          k_bghost, the stage-1 ghost copy, where a case's fills
+//                          have to run in order)
+//   k_binit                reset the per-case C-equation maxima of a stage
 //   k_bprim                primitive pass over the concatenated cells of all
 //                          cases (block ranges aligned to cases, so a block's
 //                          per-case maxima reduce to one atomicMax per warp)
@@ -13,7 +16,6 @@
 //                          and run the fused 2D RHS + RK tile of fst_mixed
 //                          (fst_batch_dev.cuh; instantiated per tile width in
 //                          fst_batch_w16/w32/w64.cu)
-//   k_bghost               stage-1 ghost copy
 // A whole time step is captured once into a CUDA graph and replayed.  The
 // RHS tile shape (width x height threads) and the persistent blocks per SM
 // are picked by an autotuner that times every candidate on the actual
@@ -59,11 +61,40 @@ const void* brhs_kernel(int w, int h, int nv) {
   }
 }
 
-__global__ void k_binit(const BCase* __restrict__ cs, int n) {
+// reset the C-equation maxima of one stage
+__global__ void k_binit(const BCase* __restrict__ cs, int n, int stage) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < n) {
-    cs[c].red[0] = FST_KEY_LOWEST;
-    cs[c].red[1] = FST_KEY_LOWEST;
+    cs[c].red[2 * (stage - 1)] = FST_KEY_LOWEST;
+    cs[c].red[2 * (stage - 1) + 1] = FST_KEY_LOWEST;
+  }
+}
+
+// The ghost rows (COLS = false: ghost in j) or ghost columns (the rest) of every
+// case, straight from interior cells (fstbc::GhostRule), into both stage buffers:
+// grid.y = case, grid.z = chunk of VC variables.
+constexpr int VC = 5;
+template <bool COLS>
+__global__ void __launch_bounds__(128) k_bfill(const BCase* __restrict__ cs) {
+  const BCase& B = cs[blockIdx.y];
+  const Geo& g = B.g;
+  const int rows = 2 * g.ng * g.ngi, cols = 2 * g.ng * g.ncj;  // fst_shell_cell's order
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= (COLS ? cols : rows)) return;
+  int i, j, k;
+  fst_shell_cell(g, COLS ? rows + t : t, i, j, k);
+  const long long dst = fst_idx(g, i, j, k);
+  const fstbc::GhostSource s = fstbc::ghost_source(g, B.rule, i, j, k);
+  const int v0 = blockIdx.z * VC;
+#pragma unroll
+  for (int q = 0; q < VC; ++q) {
+    const int v = v0 + q;
+    if (v >= g.nvt) break;
+    const double y = s.layer >= 0 && v == g.ndim
+                         ? fstbc::ghost_energy(g, B.Ua, s)
+                         : fstbc::ghost_value(B.Ua[s.src + g.sv * v], s.flip, v);
+    B.Ua[dst + g.sv * v] = y;
+    B.Ub[dst + g.sv * v] = y;
   }
 }
 
@@ -89,10 +120,11 @@ __global__ void k_bface(const BCase* __restrict__ cs, int axis, int side, bool u
 }
 
 // primitive pass: block b belongs to case find_case(block_off, b)
+template <int NS>
 __global__ void __launch_bounds__(256) k_bprim(const BCase* __restrict__ cs,
                                                const Phys* __restrict__ Ps,
                                                const int* __restrict__ block_off, int ncase,
-                                               bool use_a, bool red) {
+                                               int stage, bool red) {
   const int c = find_case(block_off, ncase, blockIdx.x);
   const BCase& B = cs[c];
   const Geo& g = B.g;
@@ -100,15 +132,15 @@ __global__ void __launch_bounds__(256) k_bprim(const BCase* __restrict__ cs,
   float lS = -3.0e38f, lC = -3.0e38f;
   if (local < (int)g.sv) {
     const int i = local % g.ngi, j = local / g.ngi;
-    mprim_cell<2>(g, g, Ps[c], use_a ? B.Ua : B.Ub, B.Q, B.rho32, B.rho64, B.vel32, B.p64, nullptr, nullptr,
+    mprim_cell<2, NS>(g, g, Ps[c], stage == 1 ? B.Ua : B.Ub, B.Q, B.rho32, B.rho64, B.vel32, B.p64, nullptr, nullptr,
                   B.nrg, B.C, B.T32, B.lo, red, i, j, 0, lS, lC);
   }
   if (red) {
     lS = warp_maxf(lS);
     lC = warp_maxf(lC);
     if ((threadIdx.x & 31) == 0 && lS > -1e38f) {
-      atomicMax(&B.red[0], fst_key((double)lS));
-      atomicMax(&B.red[1], fst_key((double)lC));
+      atomicMax(&B.red[2 * (stage - 1)], fst_key((double)lS));
+      atomicMax(&B.red[2 * (stage - 1) + 1], fst_key((double)lC));
     }
   }
 }
@@ -147,6 +179,9 @@ struct fst_batch {
   int bps = 0, bps_max = 0;  // in use; the occupancy limit of the shape
   const void* rhs = nullptr;
   int max_lines = 0, max_face = 0;
+  bool direct = true;  // every case's ghosts come straight from interior cells
+  cudaStream_t side[2] = {nullptr, nullptr};  // capture: branches of the step graph
+  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   int persistent_blocks = 0;
   int tune_candidates = 0;
   double tune_best_ms = 0.0, tune_worst_ms = 0.0;
@@ -234,17 +269,47 @@ int enqueue_step(fst_batch* b) {
       }
   };
   const bool ceq = b->cfgs[0].ceq != 0;
-  bcs(true);  // cart2d_func::preStep
-  for (int stage = 1; stage <= 2; ++stage) {
-    const bool use_a = stage == 1;
-    if (ceq) {
-      k_binit<<<cdivu(n, 64), 64, 0, b->stream>>>(b->dcases, n);
-      ++L;
+  // preStep (cart2d_func) and the resets: independent of one another, so they are
+  // branches of the graph where the fills are direct
+  auto init = [&](int stage, cudaStream_t st) {
+    if (!ceq) return;
+    k_binit<<<cdivu(n, 64), 64, 0, st>>>(b->dcases, n, stage);
+    ++L;
+  };
+  if (b->direct) {
+    const unsigned nz = cdivu(b->nvt, VC), nb = cdivu(6LL * b->max_lines, 128);
+    cudaEventRecord(b->fork, b->stream);
+    for (int q = 0; q < 2; ++q) cudaStreamWaitEvent(b->side[q], b->fork, 0);
+    k_bfill<false><<<dim3(nb, n, nz), 128, 0, b->stream>>>(b->dcases);
+    k_bfill<true><<<dim3(nb, n, nz), 128, 0, b->side[0]>>>(b->dcases);
+    L += 2;
+    init(1, b->side[1]);
+    init(2, b->side[1]);
+    for (int q = 0; q < 2; ++q) {
+      cudaEventRecord(b->join[q], b->side[q]);
+      cudaStreamWaitEvent(b->stream, b->join[q], 0);
     }
-    k_bprim<<<b->nblocks, 256, 0, b->stream>>>(b->dcases, b->dphys, b->dblock_off, n, use_a, ceq);
+  } else {
+    bcs(true);
+    init(1, b->stream);
+    init(2, b->stream);
+  }
+  for (int stage = 1; stage <= 2; ++stage) {
+    const dim3 grid(b->nblocks);
+    auto prim = [&](auto kernel) {
+      kernel<<<grid, 256, 0, b->stream>>>(b->dcases, b->dphys, b->dblock_off, n, stage, ceq);
+    };
+    switch (b->geos[0].ns) {
+      case 1: prim(k_bprim<1>); break;
+      case 2: prim(k_bprim<2>); break;
+      case 3: prim(k_bprim<3>); break;
+      case 4: prim(k_bprim<4>); break;
+      case 5: prim(k_bprim<5>); break;
+      default: prim(k_bprim<0>); break;
+    }
     ++L;
     L += enqueue_rhs(b, stage);
-    if (stage == 1) {
+    if (stage == 1 && !b->direct) {
       k_bghost<<<b->nblocks, 256, 0, b->stream>>>(b->dcases, b->dblock_off, n);
       ++L;
     }
@@ -338,6 +403,12 @@ int fst_batch_create(const fst_config* cfgs, int ncases, fst_batch** out) {
   }
   b->own_stream = true;
   int rc = FST_OK;
+  for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+    e = cudaStreamCreateWithFlags(&b->side[q], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[q], cudaEventDisableTiming);
+  }
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+  if (e != cudaSuccess) rc = bfail(b, FST_ERR_CUDA, cudaGetErrorString(e));
   std::vector<int> boff(ncases + 1, 0);
   for (int c = 0; c < ncases && !rc; ++c) {
     const Geo& g = b->geos[c];
@@ -350,7 +421,7 @@ int fst_batch_create(const fst_config* cfgs, int ncases, fst_batch** out) {
     };
     A((void**)&B.Ua, sizeof(double) * n * g.nvt);
     A((void**)&B.Ub, sizeof(double) * n * g.nvt);
-    A((void**)&B.red, sizeof(unsigned long long) * 2);
+    A((void**)&B.red, sizeof(unsigned long long) * 4);
     A((void**)&B.Q, sizeof(float) * n * g.nv);
     A((void**)&B.rho32, sizeof(float) * n);
     A((void**)&B.vel32, sizeof(float) * n * 2);
@@ -369,6 +440,8 @@ int fst_batch_create(const fst_config* cfgs, int ncases, fst_batch** out) {
     B.bc[3] = cf.bc_ymax;
     B.per[0] = cf.xper != 0;
     B.per[1] = cf.yper != 0;
+    B.rule = fstbc::ghost_rule(g, cf);
+    b->direct = b->direct && B.rule.direct && 6LL * std::max(g.ngi, g.ngj) < (1LL << 31);
     b->hcases.push_back(B);
     boff[c + 1] = boff[c] + (int)((n + 255) / 256);
     b->max_lines = std::max(b->max_lines, std::max(g.ngi, g.ngj));
@@ -408,6 +481,11 @@ void fst_batch_destroy(fst_batch* b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
   if (b->graph) cudaGraphDestroy(b->graph);
   for (void* p : b->allocs) cudaFree(p);
+  for (int q = 0; q < 2; ++q) {
+    if (b->side[q]) cudaStreamDestroy(b->side[q]);
+    if (b->join[q]) cudaEventDestroy(b->join[q]);
+  }
+  if (b->fork) cudaEventDestroy(b->fork);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }

@@ -15,12 +15,13 @@ struct BCase {
   Geo g;
   MixedView M;
   double *Ua, *Ub;
-  unsigned long long* red;  // 2 keys
+  unsigned long long* red;  // 2 keys per stage
   float* Q;                 // writable views of the mixed buffers
   float *rho32, *vel32, *T32, *nrg, *C, *lo;
   double *p64, *rho64;
   int bc[4];     // xmin, xmax, ymin, ymax
   int per[2];    // x, y periodic
+  fstbc::GhostRule rule;
 };
 
 __device__ __forceinline__ int find_case(const int* __restrict__ off, int n, int x) {
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(TXX * TYY) k_brhs(const BCase* __restrict__ cs
     const int ntx = (B.g.nci + TXX - 2) / (TXX - 1);
     const int local = w - tile_off[c];
     // stage 1: Ub = Ua + hdt*R(Ua); stage 2: Ua = Ua + dt*R(Ub)
-    rhs2d_tile<NV, false, TYY, TXX>(B.g, P, B.M, B.red, nullptr, B.Ua, stage == 1 ? B.Ub : B.Ua,
+    rhs2d_tile<NV, false, TYY, TXX>(B.g, P, B.M, B.red + 2 * (stage - 1), nullptr, B.Ua, stage == 1 ? B.Ub : B.Ua,
                                     stage == 1 ? P.hdt : P.dt, nullptr, local % ntx, local / ntx,
                                     sG, sE);
     __syncthreads();

@@ -32,7 +32,7 @@
 namespace {
 using namespace fstm;
 
-template <int NDIM>
+template <int NDIM, int NS>
 __global__ void __launch_bounds__(256) k_mprim(Geo g, Geo gq, Phys P, const double* __restrict__ U,
                                                float* __restrict__ Q, float* __restrict__ rho,
                                                double* __restrict__ rho64,
@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(256) k_mprim(Geo g, Geo gq, Phys P, const doub
   const int j = t / g.ngi, i = t - j * g.ngi;
   float lS = -3.0e38f, lC = -3.0e38f;
   if (j < g.ngj)
-    mprim_cell<NDIM>(g, gq, P, U, Q, rho, rho64, vel, pr, pp, mu, nrg, Cc, T, lo, red != nullptr, i, j,
+    mprim_cell<NDIM, NS>(g, gq, P, U, Q, rho, rho64, vel, pr, pp, mu, nrg, Cc, T, lo, red != nullptr, i, j,
                      blockIdx.z, lS, lC);
   if (red) {
     lS = warp_maxf(lS);
@@ -220,8 +220,17 @@ void launch_mprim(const Geo& g, const Geo& gq, const Phys& P, const double* U, f
                   float* nrg, float* Cc, float* T, float* lo, unsigned long long* red,
                   cudaStream_t st) {
   const dim3 qg(cdiv((long long)g.ngi * g.ngj, 256), 1, g.ngk), qb(256);
-  k_mprim<NDIM><<<qg, qb, 0, st>>>(g, gq, P, U, Q, rho, rho64, vel, pr, pp, mu, nrg, Cc, T, lo,
-                                   red);
+  auto run = [&](auto kernel) {
+    kernel<<<qg, qb, 0, st>>>(g, gq, P, U, Q, rho, rho64, vel, pr, pp, mu, nrg, Cc, T, lo, red);
+  };
+  switch (g.ns) {
+    case 1: run(k_mprim<NDIM, 1>); break;
+    case 2: run(k_mprim<NDIM, 2>); break;
+    case 3: run(k_mprim<NDIM, 3>); break;
+    case 4: run(k_mprim<NDIM, 4>); break;
+    case 5: run(k_mprim<NDIM, 5>); break;
+    default: run(k_mprim<NDIM, 0>); break;
+  }
 }
 
 Prim3Out prim3_out(const Phys& P, const MixedBufs& b, bool all_outputs) {

@@ -135,7 +135,7 @@ __device__ __forceinline__ float warp_maxf(float v) {
 // The pressure goes out as FP64 (pr) or as an FP32 pair hi + lo (pp[q],
 // pp[q + qv]) that carries ~48 bits: differences of neighbouring pressures
 // then come out of FP32 arithmetic (hi - hi' is exact for close values).
-template <int NDIM>
+template <int NDIM, int NS = 0>
 __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Phys& P,
                                            const double* __restrict__ U, float* __restrict__ Q,
                                            float* __restrict__ rho, double* __restrict__ rho64,
@@ -148,14 +148,29 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
   const long long c = (long long)i + g.sy * j + g.sz * k;
   const long long q = (long long)i + gq.sy * j + gq.sz * k;
   const int s0 = NDIM + 1;  // first species index
+  // the cell's state, every load in flight before the first use (NS species known
+  // at compile time), or loaded where it is used (NS = 0)
+  double us[NS > 0 ? NS : 1], um[NDIM + 1], uc[5];
+  if (NS > 0) {
+#pragma unroll
+    for (int s = 0; s < NS; ++s) us[s] = U[c + sv * (s0 + s)];
+#pragma unroll
+    for (int d = 0; d <= NDIM; ++d) um[d] = U[c + sv * d];
+    if (Cc) {
+#pragma unroll
+      for (int n = 0; n < 5; ++n) uc[n] = U[c + sv * (P.nv + n)];
+    }
+  }
+  auto species = [&](int s) { return NS > 0 ? us[s] : U[c + sv * (s0 + s)]; };
+  auto momentum = [&](int d) { return NS > 0 ? um[d] : U[c + sv * d]; };  // NDIM: the energy
+  const int ns = NS > 0 ? NS : P.ns;
   // mixture EOS (calculateRhoPT, src/secondary.hpp:60-151)
-  // The species loop stays rolled: unrolling it (all loads issued up front)
-  // measured 1.5x slower for this streaming pass on GB300, as did forming
-  // the two sums in double-float on the FP32 pipe.
   double sCv = 0.0, sRm = 0.0, r64 = 0.0;
   float rf = 0.f;
-  for (int s = 0; s < P.ns; ++s) {
-    const double rs = U[c + sv * (s0 + s)];
+#pragma unroll
+  for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
+    if (NS == 0 && s >= ns) break;
+    const double rs = species(s);
     if (rho64) r64 += rs;
     sCv = fma(rs, P.cv_s[s], sCv);
     sRm = fma(rs, P.rm_s[s], sRm);
@@ -164,8 +179,10 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
   const float rif = __frcp_rn(rf);
   const double gm1 = sRm * rcp64(sCv);
   float Cv2 = 0.f, Cp2 = 0.f, m = 0.f;
-  for (int s = 0; s < P.ns; ++s) {
-    const float rs = d2f(U[c + sv * (s0 + s)]);
+#pragma unroll
+  for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
+    if (NS == 0 && s >= ns) break;
+    const float rs = d2f(species(s));
     const float ys = rs * rif;
     if (NDIM == 2) {
       Cv2 += ys * P.cv2_f[s];
@@ -178,14 +195,14 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
   float msq = 0.f, usq = 0.f;
 #pragma unroll
   for (int d = 0; d < NDIM; ++d) {
-    const float mf = d2f(U[c + sv * d]);
+    const float mf = d2f(momentum(d));
     msq += mf * mf;
     const float u = mf * rif;
     usq += u * u;
     vel[q + qv * d] = u;
     Q[q + qv * d] = mf;
   }
-  const double E = U[c + sv * NDIM];
+  const double E = momentum(NDIM);
   const double p = gm1 * (E - f2d(0.5f * msq * rif));  // FP64 pressure recovery
   if (pr) pr[q] = p;
   if (pp) {
@@ -203,11 +220,15 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
     // replace the FP32 values above), for the shock and contact switches;
     // lo = [rho, nrg, u, v] low parts (see Prim3Out)
     f2p r = {0.f, 0.f};
-    for (int s = 0; s < P.ns; ++s) r = df_add(r, split(U[c + sv * (s0 + s)]));
+#pragma unroll
+    for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
+      if (NS == 0 && s >= ns) break;
+      r = df_add(r, split(species(s)));
+    }
     f2p m2 = {0.f, 0.f};
 #pragma unroll
     for (int d = 0; d < NDIM; ++d) {
-      const f2p md = split(U[c + sv * d]);
+      const f2p md = split(momentum(d));
       const f2p u = df_div(md, r);
       vel[q + qv * d] = u.h;
       lo[q + qv * (2 + d)] = u.l;
@@ -220,8 +241,15 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
     nrg[q] = e.h;
     lo[q + qv] = e.l;
   }
-  if (Cc)
-    for (int n = 0; n < 5; ++n) Cc[q + qv * n] = d2f(U[c + sv * (P.nv + n)]);
+  float chat = 0.f;
+  if (Cc) {
+#pragma unroll
+    for (int n = 0; n < 5; ++n) {
+      const float cf = d2f(NS > 0 ? uc[n] : U[c + sv * (P.nv + n)]);
+      Cc[q + qv * n] = cf;
+      if (n == 1) chat = cf;
+    }
+  }
   if (red) {
     const bool in = i >= g.ng && i < g.ngi - g.ng && j >= g.ng && j < g.ngj - g.ng &&
                     (NDIM == 2 || (k >= g.ng && k < g.ngk - g.ng));
@@ -231,7 +259,7 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
       if (NDIM == 3) sp = sqrtf((1.0f + d2f(gm1)) * pf * rif) + mf * rif;
       else sp = sqrtf(Cp2 / Cv2 * pf * rif) + mf;  // maxWaveSpeed2D quirks
       lS = fmaxf(lS, sp);
-      lC = fmaxf(lC, fabsf(Cc[q + qv]));
+      lC = fmaxf(lC, fabsf(chat));
     }
   }
 }
