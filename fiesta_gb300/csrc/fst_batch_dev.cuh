@@ -38,8 +38,11 @@ __device__ __forceinline__ int find_case(const int* __restrict__ off, int n, int
 // persistent RHS + RK stage over the (case, tile) work list: block b takes
 // work items b, b + gridDim.x, ...; item w is tile w - tile_off[c] of case c
 // (tiles of a case in row-major order, (nci + TXX - 2) / (TXX - 1) per row).
+// Bound by the latency of the tile's gathers.  1280 threads per SM (48 registers):
+// the 24-case, 1.5 M cell step takes 543 us, 554 at 1024 threads, 703 with the
+// registers the two faces' loads would take (768 threads).
 template <int NV, int TYY, int TXX>
-__global__ void __launch_bounds__(TXX * TYY) k_brhs(const BCase* __restrict__ cs,
+__global__ void __launch_bounds__(TXX * TYY, NV <= 8 ? 1280 / (TXX * TYY) : 1) k_brhs(const BCase* __restrict__ cs,
                                                     const Phys* __restrict__ Ps,
                                                     const int* __restrict__ tile_off, int ncase,
                                                     int stage) {

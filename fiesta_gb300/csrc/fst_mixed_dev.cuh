@@ -464,26 +464,39 @@ __device__ __forceinline__ bool smooth_at(const unsigned char* map, long long c,
 // 2D face terms of cart2d (src/flux.hpp:23-106, src/viscosity.hpp:25-199,
 // src/ceq.hpp:200-293) with their quirks, in FP32.
 // ---------------------------------------------------------------------------
+// WENO fluxes of the faces at (cx + 1/2, .) and (., cy + 1/2), both at once and
+// without a branch, so that the loads of one are in flight while the other's are
+// used (a face out of range is given a clamped cell and dropped by the caller).
 template <int NV, bool HYB>
-__device__ __forceinline__ void face2d(const Geo& g, const Phys& P, const MixedView& M,
-                                       const FaceCtx& fc, long long c, int f, bool smooth,
-                                       int nv, float* G) {
+__device__ __forceinline__ void faces2d_weno(const Geo& g, const MixedView& M, const FaceCtx& fc,
+                                             long long c, bool smx, bool smy, int nv, float* Gx,
+                                             float* Gy) {
+  const long long sv = g.sv, sy = g.sy;
+  const float* u = M.vel;
+  const float* v = M.vel + sv;
+  const float ux = (-u[c + 2] + 7.0f * u[c + 1] + 7.0f * u[c] - u[c - 1]) * (1.0f / 12.0f);
+  const float uy = (-v[c + 2 * sy] + 7.0f * v[c + sy] + 7.0f * v[c] - v[c - sy]) * (1.0f / 12.0f);
+  const long long cx = ux < 0.0f ? c + 3 : c - 2, ox = ux < 0.0f ? -1 : 1;
+  const long long cy = uy < 0.0f ? c + 3 * sy : c - 2 * sy, oy = uy < 0.0f ? -sy : sy;
+  const float sx_ = ux * fc.rd[0], sy_ = uy * fc.rd[1];
+#pragma unroll
+  for (int w = 0; w < NV; ++w) {
+    if (NV == NVMAX && w >= nv) break;
+    const float* q = M.Q + sv * w;
+    const float a1 = __ldg(q + cx), a2 = __ldg(q + cx + ox), a3 = __ldg(q + cx + 2 * ox),
+                a4 = __ldg(q + cx + 3 * ox), a5 = __ldg(q + cx + 4 * ox);
+    const float b1 = __ldg(q + cy), b2 = __ldg(q + cy + oy), b3 = __ldg(q + cy + 2 * oy),
+                b4 = __ldg(q + cy + 3 * oy), b5 = __ldg(q + cy + 4 * oy);
+    Gx[w] = sx_ * ((HYB && smx) ? upwind5_f(a1, a2, a3, a4, a5) : weno_f(a1, a2, a3, a4, a5));
+    Gy[w] = sy_ * ((HYB && smy) ? upwind5_f(b1, b2, b3, b4, b5) : weno_f(b1, b2, b3, b4, b5));
+  }
+}
+
+// The viscous and C-equation terms of one face, added to its fluxes G.
+__device__ __forceinline__ void face2d_terms(const Geo& g, const Phys& P, const MixedView& M,
+                                             const FaceCtx& fc, long long c, int f, float* G) {
   const long long sv = g.sv, sx = 1, sy = g.sy;
   const long long sf = f == 0 ? sx : sy;
-  const float* un = M.vel + sv * f;
-  const float uf = (-un[c + 2 * sf] + 7.0f * un[c + sf] + 7.0f * un[c] - un[c - sf]) * (1.0f / 12.0f);
-  const bool neg = uf < 0.0f;
-  const long long c0 = neg ? c + 3 * sf : c - 2 * sf;
-  const long long o = neg ? -sf : sf;
-  const float scale = uf * fc.rd[f];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (NV == NVMAX && v >= nv) break;
-    const float* q = M.Q + sv * v;
-    const float f1 = __ldg(q + c0), f2 = __ldg(q + c0 + o), f3 = __ldg(q + c0 + 2 * o),
-                f4 = __ldg(q + c0 + 3 * o), f5 = __ldg(q + c0 + 4 * o);
-    G[v] = scale * ((HYB && smooth) ? upwind5_f(f1, f2, f3, f4, f5) : weno_f(f1, f2, f3, f4, f5));
-  }
   if (!(P.visc || P.ceq)) return;
   const float* u = M.vel;
   const float* v = M.vel + sv;
@@ -572,8 +585,17 @@ __device__ __forceinline__ void rhs2d_tile(const Geo& g, const Phys& P, const Mi
   float Gx[NV], Gy[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) Gx[v] = Gy[v] = 0.f;
-  if (fi && cj) face2d<NV, HYB>(g, P, M, fc, c, 0, HYB && smooth_at(smap, c, 0), nv, Gx);
-  if (fj && ci) face2d<NV, HYB>(g, P, M, fc, c, 1, HYB && smooth_at(smap, c, 1), nv, Gy);
+  const bool vx = fi && cj, vy = fj && ci;
+  const long long cf = (long long)min(i, g.ngi - g.ng - 1) + sy * min(j, g.ngj - g.ng - 1);
+  faces2d_weno<NV, HYB>(g, M, fc, cf, HYB && smooth_at(smap, cf, 0), HYB && smooth_at(smap, cf, 1),
+                        nv, Gx, Gy);
+  face2d_terms(g, P, M, fc, cf, 0, Gx);
+  face2d_terms(g, P, M, fc, cf, 1, Gy);
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    Gx[v] = vx ? Gx[v] : 0.f;
+    Gy[v] = vy ? Gy[v] : 0.f;
+  }
 #pragma unroll
   for (int v = 0; v < NV; ++v) sG[ty][tx][v] = Gy[v];
   if (kWarpsX > 1 && (tx & 31) == 31) {
