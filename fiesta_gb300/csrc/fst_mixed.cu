@@ -11,7 +11,7 @@
 //         C-equation terms, the wave-speed and C_hat maxima
 //
 // Per stage: k_mprim over all cells (FP64 state -> FP32 primitives + FP64
-// p, and the C-equation maxima maxS, maxCh by warp max + atomicMax), then
+// p, and the C-equation maxima maxS, maxCh by block max + atomicMax), then
 // the fused right-hand side + RK stage: in 3D the two TMA-fed kernels of
 // fst_mixed3d.cu, in 2D k_mrhs2d below (a 32x8 tile of columns; each thread
 // computes the faces at i+1/2 and j+1/2 once, the left x face by shuffle,
@@ -32,6 +32,28 @@
 namespace {
 using namespace fstm;
 
+// The maxima of lS and lC over a block of 256 threads into red[0] and red[1].
+// Cells that take no part hold -3e38.  One atomic per block and word: with one per
+// warp the same-address atomics bound the whole pass at 256^3 (k_mprim3<5>: 1530 us,
+// one per block 783 us at 4.8 TB/s).
+__device__ __forceinline__ void block_max_256(unsigned long long* red, float lS, float lC) {
+  __shared__ float sS[8], sC[8];
+  lS = warp_maxf(lS);
+  lC = warp_maxf(lC);
+  if ((threadIdx.x & 31) == 0) {
+    sS[threadIdx.x >> 5] = lS;
+    sC[threadIdx.x >> 5] = lC;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    const float* v = threadIdx.x ? sC : sS;
+    float m = v[0];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) m = fmaxf(m, v[w]);
+    if (m > -1e38f) atomicMax(&red[threadIdx.x], fst_key((double)m));
+  }
+}
+
 template <int NDIM, int NS>
 __global__ void __launch_bounds__(256) k_mprim(Geo g, Geo gq, Phys P, const double* __restrict__ U,
                                                float* __restrict__ Q, float* __restrict__ rho,
@@ -50,14 +72,7 @@ __global__ void __launch_bounds__(256) k_mprim(Geo g, Geo gq, Phys P, const doub
   if (j < g.ngj)
     mprim_cell<NDIM, NS>(g, gq, P, U, Q, rho, rho64, vel, pr, pp, mu, nrg, Cc, T, lo, red != nullptr, i, j,
                      blockIdx.z, lS, lC);
-  if (red) {
-    lS = warp_maxf(lS);
-    lC = warp_maxf(lC);
-    if ((threadIdx.x & 31) == 0 && lS > -1e38f) {
-      atomicMax(&red[0], fst_key((double)lS));
-      atomicMax(&red[1], fst_key((double)lC));
-    }
-  }
+  if (red) block_max_256(red, lS, lC);
 }
 
 // 3D: the FP64-free equation of state of mprim3_cell, same grid as k_mprim
@@ -69,14 +84,7 @@ __global__ void __launch_bounds__(256) k_mprim3(Geo g, Geo gq, Phys P,
   const int j = t / g.ngi, i = t - j * g.ngi;
   float lS = -3.0e38f, lC = -3.0e38f;
   if (j < g.ngj) mprim3_cell<NS>(g, gq, P, U, O, red != nullptr, i, j, blockIdx.z, lS, lC);
-  if (red) {
-    lS = warp_maxf(lS);
-    lC = warp_maxf(lC);
-    if ((threadIdx.x & 31) == 0 && lS > -1e38f) {
-      atomicMax(&red[0], fst_key((double)lS));
-      atomicMax(&red[1], fst_key((double)lC));
-    }
-  }
+  if (red) block_max_256(red, lS, lC);
 }
 
 // The ghost cells of the 3D primitive pass (fst_shell_cell order), one
@@ -177,14 +185,7 @@ __global__ void __launch_bounds__(256) k_mupload3(Geo g, Geo gq, Phys P,
       mprim3_vals<NS>(g, P, us, um, uc, O, (long long)i + gq.sy * j + gq.sz * k, gq.sv,
                       red != nullptr, i, j, k, lS, lC);
   }
-  if (red) {
-    lS = warp_maxf(lS);
-    lC = warp_maxf(lC);
-    if ((threadIdx.x & 31) == 0 && lS > -1e38f) {
-      atomicMax(&red[0], fst_key((double)lS));
-      atomicMax(&red[1], fst_key((double)lC));
-    }
-  }
+  if (red) block_max_256(red, lS, lC);
 }
 
 template <int NV, bool HYB>
