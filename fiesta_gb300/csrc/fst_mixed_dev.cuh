@@ -2,6 +2,7 @@
 // single-case kernels (fst_mixed.cu) and the batched 2D ensemble
 // (fst_batch.cu).  See fst_mixed.cu for the design.
 #pragma once
+#include "fst_conv.cuh"
 #include "fst_internal.h"
 
 namespace fstm {
@@ -14,37 +15,6 @@ constexpr int NVMAX = 4 + FST_MAX_SPECIES;
 // ---------------------------------------------------------------------------
 // primitives
 // ---------------------------------------------------------------------------
-// FP64 <-> FP32 conversions on the integer pipe.  GB300's FP64 unit also
-// executes the F2F conversions, at the FP64 rate; these rebias the exponent
-// and round the mantissa with integer operations instead.  Values outside
-// the FP32 normal range go to signed zero / infinity (no FP32 denormals);
-// NaN stays NaN; mantissa ties round away from zero.
-__device__ __forceinline__ float d2f(double x) {
-  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
-  // the low 9 exponent bits and 23 mantissa bits in one funnel shift, then
-  // the exponent rebiased 1023 -> 127 (exact modulo 2^32 for the normal
-  // range) and the dropped bits rounded
-  unsigned int bits = __funnelshift_l(lo, hi, 3) - (896u << 23);
-  bits += (lo >> 28) & 1u;  // a carry rounds into the exponent
-  // outside the FP32 normal range (selects, no branch: zeros are common)
-  const unsigned int ex = (hi >> 20) & 0x7FFu;
-  const unsigned int big = (ex == 0x7FFu && ((hi & 0xFFFFFu) | lo)) ? 0x7FC00000u : 0x7F800000u;
-  bits = ex < 897u ? 0u : bits;
-  bits = ex > 1150u ? big : bits;
-  return __uint_as_float((hi & 0x80000000u) | bits);
-}
-__device__ __forceinline__ double f2d(float x) {
-  const unsigned int f = __float_as_uint(x), a = f & 0x7FFFFFFFu;
-  unsigned int hi = (a >> 3) + (896u << 20), lo = f << 29;  // exponent rebiased 127 -> 1023
-  // zero / FP32 denormal, inf / NaN (selects, no branch)
-  const unsigned int m = a & 0x7FFFFFu;
-  const unsigned int special = 0x7FF00000u | (m >> 3) | (m ? 0x80000u : 0u);
-  hi = a >= 0x7F800000u ? special : hi;
-  hi = a < 0x00800000u ? 0u : hi;
-  lo = a < 0x00800000u ? 0u : lo;
-  return __hiloint2double((int)(hi | (f & 0x80000000u)), (int)lo);
-}
-
 // FP64 reciprocal by one Newton-Raphson step from the correctly rounded FP32
 // reciprocal: relative error below ~1e-14 (the square of the seed's 2^-24),
 // for arguments inside the FP32 range, which holds for the densities and heat
@@ -63,9 +33,6 @@ __device__ __forceinline__ double rcp64(double x) {
 // quotient (Dekker 1971).  The rounded operations are written as intrinsics
 // so that no contraction or fast-math rewrite can change them.
 // ---------------------------------------------------------------------------
-struct f2p {
-  float h, l;
-};
 __device__ __forceinline__ f2p two_sum(float a, float b) {
   const float s = __fadd_rn(a, b);
   const float bb = __fsub_rn(s, a);
@@ -95,26 +62,6 @@ __device__ __forceinline__ f2p df_div(f2p a, f2p b) {
   rem = __fadd_rn(rem, __fmaf_rn(-q, b.l, a.l));
   return fast_two_sum(q, __fmul_rn(rem, r));
 }
-// x - d2f(x) as an FP32 number, by integer operations on the bits of x (no
-// FP64 instruction).  d2f keeps the top 23 mantissa bits and rounds on the
-// 29 it drops (D); the remainder is D * 2^(E-52), less 2^(E-23) when d2f
-// rounded up, E the unbiased exponent of x.  It is formed exactly as
-// F - B with B = 2^(E-23) and F = B * (1 + D / 2^29) (the 6 lowest bits of D
-// truncated: 2^-46 relative to x).  Zero when x is zero, non-finite, or so
-// small (|x| < 2^-103) or large (beyond FP32) that the pair has no low part.
-__device__ __forceinline__ float lo_part(double x) {
-  const unsigned int hi = (unsigned int)__double2hiint(x), lo = (unsigned int)__double2loint(x);
-  const unsigned int ex = (hi >> 20) & 0x7FFu;
-  const unsigned int sg = hi & 0x80000000u;
-  const unsigned int ef = (ex - 919u) << 23;  // FP32 exponent field of 2^(E-23)
-  const float B = __uint_as_float(sg | ef);
-  const float F = __uint_as_float(sg | ef | ((lo & 0x1FFFFFFFu) >> 6));
-  float r = __fsub_rn(F, B);
-  r = ((lo >> 28) & 1u) ? __fsub_rn(r, B) : r;
-  return (ex < 920u || ex > 1150u) ? 0.0f : r;
-}
-__device__ __forceinline__ f2p split(double x) { return {d2f(x), lo_part(x)}; }
-
 __device__ __forceinline__ float warp_maxf(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -274,7 +221,7 @@ struct Prim3Out {
 };
 
 // The 3D equation of state with no FP64 instruction, in FP32 pairs.  The
-// state values enter as pairs (d2f + lo_part); the density rho = sum rho_s,
+// state values enter as pairs (split); the density rho = sum rho_s,
 // the mixture sums sum rho_s cv_s and sum rho_s R_s, gamma - 1 = their
 // quotient and p = (gamma-1)(E - KE) (calculateRhoPT3D,
 // src/secondary.hpp:109-151) carry ~48 bits, the accuracy the pressure
@@ -290,20 +237,27 @@ struct Prim3Out {
 // um[0..2], energy um[3]), written to O at primitive index q (field stride
 // qv); returns the cell's wave speed |u| + c in *sp.  NS: the species count
 // when it is known at compile time (every loop then unrolls), 0 for any.
-template <int NS>
-__device__ __forceinline__ void eos3(const Phys& P, const double* us, const double um[4],
-                                     const Prim3Out& O, long long q, long long qv, float* sp) {
+template <int NS, bool RANGE>
+__device__ __forceinline__ void eos3_of(const Phys& P, const double* us, const double um[4],
+                                        const Prim3Out& O, long long q, long long qv, float* sp) {
   f2p r = {0.f, 0.f}, cv = {0.f, 0.f}, rm = {0.f, 0.f};
   float msum = 0.f;
   const int ns = NS > 0 ? NS : P.ns;
 #pragma unroll
   for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
     if (NS == 0 && s >= ns) break;
-    const f2p a = split(us[s]);
+    const f2p a = split<RANGE>(us[s]);
     O.Q[q + qv * (4 + s)] = a.h;
-    r = df_add(r, a);
-    cv = df_add(cv, df_mul(a, f2p{P.cv_f[s], P.cv_lf[s]}));
-    rm = df_add(rm, df_mul(a, f2p{P.rm_f[s], P.rm_lf[s]}));
+    const f2p c = df_mul(a, f2p{P.cv_f[s], P.cv_lf[s]}), m = df_mul(a, f2p{P.rm_f[s], P.rm_lf[s]});
+    if (RANGE && s == 0) {  // df_add to zero of a finite, for c and m normalised, pair
+      r = fast_two_sum(__fadd_rn(0.f, a.h), a.l);
+      cv = {__fadd_rn(0.f, c.h), c.l};
+      rm = {__fadd_rn(0.f, m.h), m.l};
+    } else {
+      r = df_add(r, a);
+      cv = df_add(cv, c);
+      rm = df_add(rm, m);
+    }
     msum = fmaf(a.h, P.mu_f[s], msum);
   }
   const float rif = __frcp_rn(r.h);
@@ -312,14 +266,14 @@ __device__ __forceinline__ void eos3(const Phys& P, const double* us, const doub
   float msq = 0.f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    m[d] = split(um[d]);
+    m[d] = split<RANGE>(um[d]);
     O.Q[q + qv * d] = m[d].h;
     msq = fmaf(m[d].h, m[d].h, msq);
     const f2p u = df_div(m[d], r);
     O.vel[q + qv * d] = u.h;
     if (O.lo) O.lo[q + qv * (2 + d)] = u.l;
   }
-  const f2p E = split(um[3]);
+  const f2p E = split<RANGE>(um[3]);
   const f2p gm1 = df_div(rm, cv);
   const f2p p = df_mul(gm1, df_add(E, f2p{-0.5f * msq * rif, 0.f}));
   O.pp[q] = p.h;
@@ -340,6 +294,19 @@ __device__ __forceinline__ void eos3(const Phys& P, const double* us, const doub
     }
   }
   *sp = sqrtf((1.0f + gm1.h) * p.h * rif) + sqrtf(msq) * rif;
+}
+
+// One test for the cell in place of the range selects of every split: a state with a
+// value at or beyond 2^128 (or not finite) takes the general form.
+template <int NS>
+__device__ __forceinline__ void eos3(const Phys& P, const double* us, const double um[4],
+                                     const Prim3Out& O, long long q, long long qv, float* sp) {
+  if (NS == 0) return eos3_of<0, false>(P, us, um, O, q, qv, sp);
+  unsigned int m = max(max(abs_hi(um[0]), abs_hi(um[1])), max(abs_hi(um[2]), abs_hi(um[3])));
+#pragma unroll
+  for (int s = 0; s < NS; ++s) m = max(m, abs_hi(us[s]));
+  if (m < F32_OVER_HI) eos3_of<NS, true>(P, us, um, O, q, qv, sp);
+  else eos3_of<NS, false>(P, us, um, O, q, qv, sp);
 }
 
 // One cell of the 3D primitive pass from its FP64 state values (species
