@@ -157,14 +157,21 @@ FST_HD Recip recip_of(double b) {
 // quotient's integer bits alone.
 // Measured on GB300, clocks of a sub-partition per warp: 129 (recip_of
 // included) against the operator's 601, and hidden behind two FP64 operations.
-FST_HD double div_by(double a, const Recip& b) {
+// div_exact: operands for which div_core holds (a normal or zero, b normal, the quotient
+// well inside the normal range).  Several quotients in one straight line, tested
+// together afterwards, overlap: three in turn take one warp 800 clocks, three cores 335.
+FST_HD bool div_exact(double a, const Recip& b) {
+  const uint64_t ba = bits_of(a);
+  const uint32_t ea = (uint32_t)(ba >> 52) & 0x7FFu, eb = (b.hi >> 20) & 0x7FFu;
+  const uint32_t ex = (ba << 1) == 0 ? eb : ea;
+  return !(ex - 1u >= 2046u || eb - 1u >= 2046u || ex + 1000u - eb > 2000u);
+}
+FST_HD double div_core(double a, const Recip& b) {
   const uint64_t ba = bits_of(a);
   const uint32_t ahi = (uint32_t)(ba >> 32), al = (uint32_t)ba;
   const uint32_t ea = (ahi >> 20) & 0x7FFu, eb = (b.hi >> 20) & 0x7FFu;
   const bool zero = (ba << 1) == 0;
   const uint32_t ex = zero ? eb : ea;
-  if (ex - 1u >= 2046u || eb - 1u >= 2046u || ex + 1000u - eb > 2000u)
-    return div_any(a, of_bits(((uint64_t)b.hi << 32) | b.lo));
   const uint32_t ah = (ahi & 0xFFFFFu) | 0x100000u, bh = (b.hi & 0xFFFFFu) | 0x100000u;
   const uint64_t q = quot55(ah, al, bh, b.lo, b.R);
   const uint32_t t = (uint32_t)(q >> 55);  // 1: a' >= b', 56 bits
@@ -172,6 +179,10 @@ FST_HD double div_by(double a, const Recip& b) {
   const uint32_t hi = (uint32_t)(m >> 32) + ((ex - eb + 1021u + t) << 20);
   const uint32_t sg = (ahi ^ b.hi) & 0x80000000u;
   return of_bits(((uint64_t)((zero ? 0u : hi) | sg) << 32) | (zero ? 0u : (uint32_t)m));
+}
+FST_HD double div_by(double a, const Recip& b) {
+  if (!div_exact(a, b)) return div_any(a, of_bits(((uint64_t)b.hi << 32) | b.lo));
+  return div_core(a, b);
 }
 FST_HD double div_rn(double a, double b) { return div_by(a, recip_of(b)); }
 

@@ -31,6 +31,8 @@
 
 namespace {
 using fst64::div_by;
+using fst64::div_core;
+using fst64::div_exact;
 
 constexpr int T3 = 8;   // 3D tile edge (cells)
 constexpr int T2 = 32;  // 2D tile edge
@@ -79,10 +81,10 @@ __global__ void __launch_bounds__(256) k_noise_maxabs(Geo g, const double* __res
 // the weight of term n (planes k+1, k, k-1; rows j+1, j, j-1; columns i-1,
 // i, i+1) of the 3D detection stencil: -88 at the centre, 8 on the six face
 // neighbours, 2 elsewhere
-__device__ __forceinline__ double stencil_weight(int n) {
+__device__ __forceinline__ double stencil_weight(int n, double w2 = 2.0, double w8 = 8.0) {
   const int pk = n / 9, rj = (n / 3) % 3, ci = n % 3;
-  return pk == 1 ? (rj == 1 ? (ci == 1 ? -88.0 : 8.0) : (ci == 1 ? 8.0 : 2.0))
-                 : ((rj == 1 && ci == 1) ? 8.0 : 2.0);
+  return pk == 1 ? (rj == 1 ? (ci == 1 ? -88.0 : w8) : (ci == 1 ? w8 : w2))
+                 : ((rj == 1 && ci == 1) ? w8 : w2);
 }
 
 // vars[q] without a local-memory copy of the kernel parameter
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(256) k_noise_detect(Geo g, const double* __res
   const int ii = (int)(t % cx), jj = (int)((t / cx) % cy), kk = (int)(t / ((long long)cx * cy));
   const int i = g.ng + 2 * ii, j = g.ng + 2 * jj, k = NDIM == 3 ? g.ng + 2 * kk : 0;
   unsigned hit = 0;
+  const fst64::Fused F(A.nvars);
+  const double w2 = fst64::lane_const(2.0, A.nvars), w8 = fst64::lane_const(8.0, A.nvars);
   for (int q = 0; q < A.nvars; ++q) {
     const double* var = U + g.sv * pick(A.vars, q);
     double c;
@@ -126,15 +130,18 @@ __global__ void __launch_bounds__(256) k_noise_detect(Geo g, const double* __res
         t[n] = var[(long long)(i - 1 + ci) + g.sy * (j + 1 - rj) + g.sz * (k + 1 - pk)];
         emax = max(emax, (unsigned)(fst_bits(t[n]) >> 52) & 0x7ffu);
       }
-      double sum = 2.0 * t[0];
+      double sum;
       if (emax < 1023 + 1020) {
         // every |value| < 2^1020: the weights 2 and 8 scale exactly, so
         // fma(w, v, sum) rounds sum + w*v once, as the reference's
-        // sum + (w*v) does -- the same bits for half the FP64 operations
+        // sum + (w*v) does -- the same bits for half the FP64 operations,
+        // their constants in registers (fst64::Fused)
+        sum = F.mul(w2, t[0]);
 #pragma unroll
         for (int n = 1; n < 27; ++n)
-          sum = n == 13 ? sum + -88.0 * t[n] : __fma_rn(stencil_weight(n), t[n], sum);
+          sum = n == 13 ? F.add(sum, F.mul(-88.0, t[n])) : __fma_rn(stencil_weight(n, w2, w8), t[n], sum);
       } else {
+        sum = 2.0 * t[0];
 #pragma unroll
         for (int n = 1; n < 27; ++n) sum = sum + stencil_weight(n) * t[n];
       }
@@ -182,15 +189,16 @@ __device__ __forceinline__ bool unsafe_value(double x, long long safe) {
   return (b & 0x7fffffffffffffffull) >= (unsigned long long)safe || b == 0x8000000000000000ull;
 }
 
-// OR of `bits` over the block, written by thread 0 to *out
-__device__ __forceinline__ void block_or_store(unsigned bits, int* out) {
+// OR of `bits` over the block
+__device__ __forceinline__ unsigned block_or(unsigned bits) {
   __shared__ unsigned acc;
+  __syncthreads();  // an earlier call's result has been read
   if (threadIdx.x == 0) acc = 0;
   __syncthreads();
   const unsigned w = __reduce_or_sync(0xffffffffu, bits);
   if ((threadIdx.x & 31) == 0 && w) atomicOr(&acc, w);
   __syncthreads();
-  if (threadIdx.x == 0) *out = (int)acc;
+  return acc;
 }
 
 // The tiles a removal sweep must visit, bit q for variable vars[q]: a cell
@@ -215,8 +223,13 @@ __global__ void __launch_bounds__(256) k_noise_tiles3(Geo g, const double* __res
     if (x < xe && y < ye && z < ze)
       bits |= (unsigned)noise[(long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y) + g.sz * (k0 + 1 + z)];
   }
-  bits &= (1u << R.nvars) - 1;
+  bits = block_or(bits & ((1u << R.nvars) - 1));
+  if (bits == (1u << R.nvars) - 1) {  // every variable has a flagged cell here
+    if (tid == 0) tiles[blockIdx.x] = (int)bits;
+    return;
+  }
   for (int q = 0; q < R.nvars; ++q) {
+    if ((bits >> q) & 1) continue;
     const double* var = U + g.sv * pick(R.vars, q);
     bool bad = false;
 #pragma unroll
@@ -228,7 +241,8 @@ __global__ void __launch_bounds__(256) k_noise_tiles3(Geo g, const double* __res
     }
     if (bad) bits |= 1u << q;
   }
-  block_or_store(bits, tiles + blockIdx.x);
+  bits = block_or(bits);
+  if (tid == 0) tiles[blockIdx.x] = (int)bits;
 }
 
 __global__ void __launch_bounds__(256) k_noise_tiles2(Geo g, const double* __restrict__ U,
@@ -245,8 +259,13 @@ __global__ void __launch_bounds__(256) k_noise_tiles2(Geo g, const double* __res
     const int x = p % T2, y = p / T2;
     if (x < xe && y < ye) bits |= (unsigned)noise[(long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y)];
   }
-  bits &= (1u << R.nvars) - 1;
+  bits = block_or(bits & ((1u << R.nvars) - 1));
+  if (bits == (1u << R.nvars) - 1) {  // every variable has a flagged cell here
+    if (tid == 0) tiles[blockIdx.x] = (int)bits;
+    return;
+  }
   for (int q = 0; q < R.nvars; ++q) {
+    if ((bits >> q) & 1) continue;
     const double* var = U + g.sv * pick(R.vars, q);
     bool bad = false;
 #pragma unroll
@@ -258,7 +277,8 @@ __global__ void __launch_bounds__(256) k_noise_tiles2(Geo g, const double* __res
     }
     if (bad) bits |= 1u << q;
   }
-  block_or_store(bits, tiles + blockIdx.x);
+  bits = block_or(bits);
+  if (tid == 0) tiles[blockIdx.x] = (int)bits;
 }
 
 // after a visited tile's update: if it left a value unsafe for its
@@ -269,13 +289,31 @@ __device__ __forceinline__ bool hard_value(double x, long long safe) {
   return (fst_bits(x) & 0x7fffffffffffffffull) >= (unsigned long long)safe;
 }
 
-// cells of an 8-cube with x+y+z = s, ordered by z then y: those in plane z
-// number c(s - z), c(u) = min(u, 7) - max(0, u - 7) + 1 for 0 <= u <= 14
-__device__ __forceinline__ int row_cells(int u) {
-  return u < 0 || u > 2 * T3 - 2 ? 0 : min(u, T3 - 1) - max(0, u - (T3 - 1)) + 1;
+// The 512 cells of an 8-cube (x + 8y + 64z) by wavefront x+y+z, then z, then y:
+// rank[cell] is a cell's place in that order, wavefront w holds the places
+// off[w] .. off[w+1).
+struct Waves {
+  unsigned short rank[T3 * T3 * T3];
+  short off[3 * T3 - 1];
+};
+constexpr Waves make_waves() {
+  Waves v{};
+  int n = 0;
+  for (int w = 0; w <= 3 * T3 - 3; ++w) {
+    v.off[w] = (short)n;
+    for (int z = 0; z < T3; ++z)
+      for (int y = 0; y < T3; ++y) {
+        const int x = w - y - z;
+        if (x >= 0 && x < T3) v.rank[x + T3 * y + T3 * T3 * z] = (unsigned short)n++;
+      }
+  }
+  v.off[3 * T3 - 2] = (short)n;
+  return v;
 }
+__device__ const Waves waves_rank = make_waves();    // read by consecutive threads
+__constant__ Waves waves_off = make_waves();          // read by all threads alike
 
-constexpr int R3 = 256;  // threads per 3D tile: up to three variables x 64 threads in a step
+constexpr int R3 = 160;  // threads per 3D tile: three variables' widest wavefront (3 x 48) in 5 warps
 
 // OR of per-thread bits over the block into *acc (zeroed before a barrier)
 __device__ __forceinline__ void or_into(unsigned* acc, unsigned bits) {
@@ -283,115 +321,145 @@ __device__ __forceinline__ void or_into(unsigned* acc, unsigned bits) {
   if ((threadIdx.x & 31) == 0 && w) atomicOr(acc, w);
 }
 
-// One diagonal (tx+ty+tz = diag) of 8x8x8 interior tiles.  The filtered
-// variables are swept side by side: threads 64q .. 64q+63 run variable q's
-// wavefront steps (each variable's sweep reads and writes only its own
-// values), with the cells of wavefront w in consecutive threads (a table in
-// shared memory), so a step's FP64 work occupies ceil(cells/32) warps per
-// variable rather than every warp the wavefront crosses.
-__global__ void __launch_bounds__(R3, 3) k_noise_remove3(Geo g, double* __restrict__ U,
+// One diagonal (tx+ty+tz = diag) of 8x8x8 interior tiles.  The filtered variables are
+// swept side by side (each variable's sweep reads and writes only its own values): a
+// step's cells of all of them, one after another, occupy consecutive threads, so its
+// FP64 work takes ceil(cells/32) warps.  Sums and products are fused operations
+// (fst64::Fused): 10 of the FP64 unit a cell.  What bounds the kernel is the chain of a
+// step (22 a tile, 1330 clocks each with one warp per sub-partition: eight FP64
+// operations and a division one after another), then the unit on the diagonals with
+// several tiles per SM.  The three quotients are formed side by side and tested
+// afterwards, and only the updated neighbours are read after the step's barrier.
+// A diagonal at 192^3, 3 variables: 47.9 us with 64 threads per variable (90 warps a
+// tile in place of 58), 14 operations and quotients in turn, 30.5 us now.
+// Letting the next diagonal's blocks start and load early (programmatic dependent
+// launch) made the filter slower: 2435 us against 2069 at 192^3.
+__global__ void __launch_bounds__(R3, 4) k_noise_remove3(Geo g, double* __restrict__ U,
                                                          const int* __restrict__ noise,
                                                          int* __restrict__ tiles, RemoveArgs R,
                                                          int diag, int ntx, int nty, int ntz) {
   const int tx = blockIdx.x % ntx, ty = blockIdx.x / ntx, tz = diag - tx - ty;
   if (tz < 0 || tz >= ntz) return;  // uniform over the block
   const int tile = blockIdx.x + ntx * nty * tz;
-  const unsigned cand = (unsigned)tiles[tile];
+  const unsigned cand = (unsigned)tiles[tile] & ((1u << R.nvars) - 1);
   if (!cand) return;  // no variable to visit (k_noise_tiles3)
   constexpr int E = T3 + 2, C = T3 * T3 * T3, W = 3 * T3 - 2, E3 = E * E * E;
-  __shared__ double s[3][E][E][E];       // per variable: [z][y][x], tile + one-cell halo
-  __shared__ int msk[C];                 // indicator of the tile's cells (0 outside)
-  __shared__ unsigned short order[C];    // cells (x + 8y + 64z) by wavefront
-  __shared__ short off[W + 1];           // wavefront w: order[off[w] .. off[w+1])
+  __shared__ double s[3][E3];          // per variable: [z][y][x], tile + one-cell halo
+  __shared__ unsigned short cells[C];  // by wavefront: place in s | indicator << 10, or NONE
+  constexpr unsigned short NONE = 0xFFFF;
   __shared__ unsigned busy_s, hard_s;
   const int tid = threadIdx.x;
   const int i0 = g.ng + T3 * tx - 1, j0 = g.ng + T3 * ty - 1, k0 = g.ng + T3 * tz - 1;
   const int xe = min(T3, g.ngi - g.ng - (i0 + 1)), ye = min(T3, g.ngj - g.ng - (j0 + 1)),
             ze = min(T3, g.ngk - g.ng - (k0 + 1));  // interior extent of the tile
   if (tid == 0) busy_s = hard_s = 0;
-  unsigned bits = 0;
-  for (int p = tid; p < C; p += R3) {
+  constexpr int NL = (E3 + R3 - 1) / R3;
+  constexpr int NM = (C + R3 - 1) / R3;
+  double v[3][NL];
+  int m[NM], rk[NM];
+#pragma unroll
+  for (int u = 0; u < NM; ++u) {  // every load in flight before the first store
+    const int p = tid + u * R3;
     const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3);
-    const int m = x < xe && y < ye && z < ze
-                      ? noise[(long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y) + g.sz * (k0 + 1 + z)]
-                      : 0;
-    msk[p] = m;
-    bits |= (unsigned)m;
+    rk[u] = p < C ? waves_rank.rank[p] : 0;
+    m[u] = p < C && x < xe && y < ye && z < ze
+               ? noise[(long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y) + g.sz * (k0 + 1 + z)]
+               : 0;
   }
-  for (int q = 0; q < R.nvars; ++q) {
-    if (!((cand >> q) & 1)) continue;
-    const double* var = U + g.sv * pick(R.vars, q);
-    double* sq = &s[q][0][0][0];
-    constexpr int NL = (E3 + R3 - 1) / R3;
-    double v[NL];
 #pragma unroll
-    for (int u = 0; u < NL; ++u) {  // every load in flight before the first store
-      const int p = tid + u * R3;
-      const int x = i0 + p % E, y = j0 + (p / E) % E, z = k0 + p / (E * E);
-      if (p < E3 && x < g.ngi && y < g.ngj && z < g.ngk) v[u] = var[(long long)x + g.sy * y + g.sz * z];
+  for (int u = 0; u < NL; ++u) {
+    const int p = tid + u * R3;
+    const int x = i0 + p % E, y = j0 + (p / E) % E, z = k0 + p / (E * E);
+    const long long c = (long long)x + g.sy * y + g.sz * z;
+    const bool in = p < E3 && x < g.ngi && y < g.ngj && z < g.ngk;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (in && ((cand >> q) & 1)) v[q][u] = U[c + g.sv * R.vars[q]];
+  }
+  unsigned bits = 0;
+#pragma unroll
+  for (int u = 0; u < NM; ++u) {
+    const int p = tid + u * R3;
+    if (p < C) {
+      const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3);
+      cells[rk[u]] = x < xe && y < ye && z < ze
+                         ? (unsigned short)(((z + 1) * E + y + 1) * E + x + 1 + ((m[u] & 7) << 10))
+                         : NONE;
+      bits |= (unsigned)m[u];
     }
+  }
 #pragma unroll
-    for (int u = 0; u < NL; ++u) {
-      const int p = tid + u * R3;
-      const int x = i0 + p % E, y = j0 + (p / E) % E, z = k0 + p / (E * E);
-      if (p < E3 && x < g.ngi && y < g.ngj && z < g.ngk) {
-        sq[p] = v[u];
-        if (unsafe_value(v[u], R.safe)) bits |= 1u << q;
+  for (int u = 0; u < NL; ++u) {
+    const int p = tid + u * R3;
+    const int x = i0 + p % E, y = j0 + (p / E) % E, z = k0 + p / (E * E);
+    const bool in = p < E3 && x < g.ngi && y < g.ngj && z < g.ngk;
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      if (in && ((cand >> q) & 1)) {
+        s[q][p] = v[q][u];
+        if (unsafe_value(v[q][u], R.safe)) bits |= 1u << q;
       }
-    }
   }
   __syncthreads();  // busy_s zeroed
-  or_into(&busy_s, bits & cand & ((1u << R.nvars) - 1));
+  or_into(&busy_s, bits & cand);
   __syncthreads();
   const unsigned busy = busy_s;
   if (!busy) return;
-  if (tid <= W) {  // cells with x+y+z = w ordered by z then y
-    int o = 0;
-    for (int z = 0; z < T3; ++z)
-      for (int w = 0; w < tid; ++w) o += row_cells(w - z);
-    off[tid] = (short)o;
-  }
-  __syncthreads();
-  for (int p = tid; p < C; p += R3) {
-    const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3), w = x + y + z;
-    int r = off[w] + y - max(0, w - z - (T3 - 1));
-    for (int zz = 0; zz < z; ++zz) r += row_cells(w - zz);
-    order[r] = (unsigned short)p;
-  }
-  __syncthreads();
+  const fst64::Fused F(R.nvars);
   const double D = R.dx * R.dx + R.dy * R.dy + R.dz * R.dz;
-  const int q = tid >> 6, lt = tid & 63;  // this thread's variable and lane in its group
-  const bool mine = q < R.nvars && ((busy >> q) & 1);
-  for (int w = 0; w < W; ++w) {
-    const int t = off[w] + lt;
-    if (mine && t < off[w + 1]) {
-      const int p = order[t];
-      const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3);
-      if (x < xe && y < ye && z < ze) {
-        double (*sv3)[E][E] = s[q];
-        const int a = x + 1, b = y + 1, c = z + 1;
-        const double nz = (double)((msk[p] >> q) & 1);
-        const double s2 = 2 * sv3[c][b][a];
-        const double lap = div_by(sv3[c][b][a - 1] - s2 + sv3[c][b][a + 1], R.rx) +
-                           div_by(sv3[c][b - 1][a] - s2 + sv3[c][b + 1][a], R.ry) +
-                           div_by(sv3[c - 1][b][a] - s2 + sv3[c + 1][b][a], R.rz);
-        const double dnoise = R.eta * D * nz * lap;
-        sv3[c][b][a] += dnoise;
-      }
+  const double f0 = R.eta * D * 0.0, f1 = R.eta * D * 1.0;  // eta * D * indicator
+  const int nb = __popc(busy), q0 = __ffs(busy) - 1, q2 = 31 - __clz(busy);  // busy variables in order
+  const double m2 = fst64::lane_const(-2.0, R.nvars);
+  // A thread's cell of a step.  What the steps before do not write is read a step ahead,
+  // so that only the three updated neighbours are read after the barrier.
+  struct Cell {
+    double* c;  // nullptr: none
+    double c0, xp, yp, zp, f;
+  };
+  auto cell = [&](int w) {
+    Cell k{};
+    const int o = waves_off.off[w], n = waves_off.off[w + 1] - o;
+    const int r = tid < n ? 0 : tid < 2 * n ? 1 : 2;
+    const int e = tid < nb * n ? cells[o + tid - r * n] : NONE;
+    if (e != NONE) {
+      const int q = r == 0 ? q0 : r == nb - 1 ? q2 : 1;
+      k.c = &s[q][e & 1023];
+      k.c0 = k.c[0], k.xp = k.c[1], k.yp = k.c[E], k.zp = k.c[E * E];
+      k.f = (e >> (10 + q)) & 1 ? f1 : f0;
     }
+    return k;
+  };
+  Cell k = cell(0);
+  for (int w = 0; w < W; ++w) {
+    const Cell nx = cell(w + 1 < W ? w + 1 : w);
+    if (k.c) {
+      const double xm = k.c[-1], ym = k.c[-E], zm = k.c[-E * E];
+      // -2 c0 + x as one operation: 2 c0 is exact below 2^1023
+      const double ax = F.add(__fma_rn(m2, k.c0, xm), k.xp), ay = F.add(__fma_rn(m2, k.c0, ym), k.yp),
+                   az = F.add(__fma_rn(m2, k.c0, zm), k.zp);
+      double lap = F.add(F.add(div_core(ax, R.rx), div_core(ay, R.ry)), div_core(az, R.rz));
+      const bool in = ((unsigned)(fst_bits(k.c0) >> 32) & 0x7FFFFFFFu) < 0x7FD00000u;
+      if (!(in & div_exact(ax, R.rx) & div_exact(ay, R.ry) & div_exact(az, R.rz))) {
+        const double s2 = fst64::twice(k.c0);
+        lap = div_by(xm - s2 + k.xp, R.rx) + div_by(ym - s2 + k.yp, R.ry) + div_by(zm - s2 + k.zp, R.rz);
+      }
+      k.c[0] = F.add(k.c0, F.mul(k.f, lap));
+    }
+    k = nx;
     __syncthreads();
   }
   unsigned hard = 0;
-  for (int qq = 0; qq < R.nvars; ++qq) {
-    if (!((busy >> qq) & 1)) continue;
-    double* var = U + g.sv * pick(R.vars, qq);
-    for (int p = tid; p < C; p += R3) {
-      const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3);
-      if (x < xe && y < ye && z < ze) {
-        const double val = s[qq][z + 1][y + 1][x + 1];
-        var[(long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y) + g.sz * (k0 + 1 + z)] = val;
-        if (hard_value(val, R.safe)) hard |= 1u << qq;
-      }
+  for (int p = tid; p < C; p += R3) {
+    const int x = p % T3, y = (p / T3) % T3, z = p / (T3 * T3);
+    if (x < xe && y < ye && z < ze) {
+      const long long c = (long long)(i0 + 1 + x) + g.sy * (j0 + 1 + y) + g.sz * (k0 + 1 + z);
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if ((busy >> q) & 1) {
+          const double val = s[q][((z + 1) * E + y + 1) * E + x + 1];
+          U[c + g.sv * R.vars[q]] = val;
+          if (hard_value(val, R.safe)) hard |= 1u << q;
+        }
     }
   }
   or_into(&hard_s, hard);
