@@ -28,7 +28,7 @@ DivC make_div(double d) {
   double m = std::frexp(d, &e);
   // (|k| <= 1000: scale2's range; a wilder spacing takes the division)
   q.inv = (d > 0.0 && m == 0.5 && e > -1000 && e < 1000) ? 1.0 / d : 0.0;
-  q.k = 1 - e;  // d = 2^(e-1)
+  q.k = q.inv != 0.0 ? 1 - e : DivC::NONE;  // d = 2^(e-1)
   q.r = fst64::recip_of(d);
   return q;
 }

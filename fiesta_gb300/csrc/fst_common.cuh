@@ -26,14 +26,16 @@ struct Geo {
 // bit-identical to a/d either way.
 struct DivC {
   double d, inv;  // inv = 1/d if d is a power of two, else 0
-  int k;          // inv = 2^k
+  int k;          // inv = 2^k, or NONE: tested in place of inv, whose compare would take the
+                  // FP64 unit as long as a sum (k_cell3d at 256^3: 10.1 ms against 8.2)
   fst64::Recip r;
+  static constexpr int NONE = 1 << 20;
   __device__ __forceinline__ double operator()(double a) const {
-    return inv != 0.0 ? fst64::scale2(a, k, inv) : fst64::div_by(a, r);
+    return k != NONE ? fst64::scale2(a, k, inv) : fst64::div_by(a, r);
   }
   // the same with the division as a call (fst64::div_call)
   __device__ __forceinline__ double call(double a) const {
-    return inv != 0.0 ? fst64::scale2(a, k, inv) : fst64::div_call(a, r.hi, r.lo, r.R);
+    return k != NONE ? fst64::scale2(a, k, inv) : fst64::div_call(a, r.hi, r.lo, r.R);
   }
 };
 

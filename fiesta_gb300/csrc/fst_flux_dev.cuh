@@ -19,8 +19,9 @@
 //
 // Measured at 256^3, 9 variables, dx a power of two (per stage): 93.5 ms as one
 // thread per face index with the operators, 49.5 with shared cell terms, fused
-// forms and integer divisions, 25.3 with the products and sums as well: FP64
-// unit 85 % busy, integer unit 52 %, 1240 instructions per face and variable.
+// forms and integer divisions, 25.3 with the products and sums as well, 23.1 with
+// no compare or predicated-off operation left on the FP64 unit (either takes as long
+// as a sum): unit 82 % busy, integer unit 55 %, 44 instructions per FP64 one.
 #pragma once
 #include "fst_internal.h"
 
@@ -131,6 +132,10 @@ __device__ __forceinline__ double weno_core(const FK& k, double f1, double f2, d
   return div_rn(k.add(k.add(wp(w1, p1), wp(w2, p2)), wp(w3, p3)), k.add(k.add(w1, w2), w3));
 }
 
+// x + p of the energy's stencil values, out of line: one warp in nv needs it, and
+// inlined it would be predicated and take the FP64 unit's time for the others too
+__device__ __noinline__ static double add_apart(double x, double p) { return x + p; }
+
 // One direction's share of the flux launch: lines of `n` interior cells along
 // the direction, `lines` of them (na x nb interior transverse cells), cut into
 // `nseg` segments of at most LSEG faces.
@@ -203,7 +208,7 @@ __global__ void __launch_bounds__(32 * WMAX, 4)
     // where it is not.
     auto value = [&](long long o) {
       const double x = q[o], p = pq[o];
-      if (v == ve) return k.add(x, p);
+      if (v == ve) return add_apart(x, p);
       return fst_finite(p) ? x : fst64::of_bits(0x7FF8000000000000ull);
     };
     // outside weno_core's range: not 0 and not in [2^-200, 2^150)

@@ -328,9 +328,10 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
                       12.0);
       };
       const double d = k.add(k.add(d4m(sx, 0), d4m(sy, 1)), d4m(sz, 2));
-      if (w == 0) R0 = k.sub(R0, d);
-      else if (w == 1) R1 = k.sub(R1, d);
-      else R2 = k.sub(R2, d);
+      const double R = k.sub(w == 0 ? R0 : w == 1 ? R1 : R2, d);  // one operation, not three predicated
+      if (w == 0) R0 = R;
+      else if (w == 1) R1 = R;
+      else R2 = R;
     }
   } else {  // pressure gradient; the reference uses dz = cd(2) for the z term
 #pragma unroll 1
@@ -338,9 +339,10 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
       const long long s = stride(f);
       const DivC& d12 = f == 2 ? P.d12pz : P.d12[f];
       const double d = d12.call(d4sum(pr[c - 2 * s], pr[c - s], pr[c + s], pr[c + 2 * s]));
-      if (f == 0) R0 = k.sub(R0, d);
-      else if (f == 1) R1 = k.sub(R1, d);
-      else R2 = k.sub(R2, d);
+      const double R = k.sub(f == 0 ? R0 : f == 1 ? R1 : R2, d);  // one operation, not three predicated
+      if (f == 0) R0 = R;
+      else if (f == 1) R1 = R;
+      else R2 = R;
     }
   }
   if (P.buoyancy) {
