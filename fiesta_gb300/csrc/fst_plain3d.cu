@@ -123,7 +123,12 @@ __global__ void __launch_bounds__(256, 5) k_prim3d(Geo g, Phys P, const double* 
 // (fst_fp64.cuh), products and divisions as calls.  Measured at 192^3, 5 species,
 // per launch: 6.4 ms with all of it inlined (the warps wait for instructions),
 // 4.34 with calls, 3.74 at 7 blocks per SM instead of 5, 3.49 with 12 of a face's
-// products on the FP64 unit, which then is as busy as the integer one.
+// products on the FP64 unit, which then is as busy as the integer one.  A plane's
+// faces are numbered row after row, so that warps are full for any row length (rows
+// cut into warps of 32 left a fifth of the unit idle at 100 or 129 faces a row): step
+// at 100^3, 3 species, 3683 -> 3467 us with this pass and k_cell3d so numbered, at
+// 64^3 1516 -> 1485; where rows are multiples of 32 the cell pass loses 0.8 % (rows
+// above and below no longer share a block), the step nothing.
 // ---------------------------------------------------------------------------
 template <int F>
 __device__ __forceinline__ void face_terms3d(const Geo& g, const Phys& P, const fst64::Fused& k,
@@ -197,11 +202,12 @@ __global__ void __launch_bounds__(128, 7) k_faces3d(Geo g, Phys P, const double*
                                                  const unsigned long long* __restrict__ red,
                                                  double* __restrict__ S, double* __restrict__ MF) {
   const int f = blockIdx.x % 3;
-  // faces c + 1/2 along f for c from the last ghost, interior cells across
-  const int i = g.ng - (f == 0) + blockIdx.x / 3 * blockDim.x + threadIdx.x;
-  const int j = g.ng - (f == 1) + blockIdx.y * blockDim.y + threadIdx.y;
+  // faces c + 1/2 along f for c from the last ghost, interior cells across, row after row
+  const int t = blockIdx.x / 3 * 128 + threadIdx.x, nx = g.nci + (f == 0), r = t / nx;
+  const int i = g.ng - (f == 0) + t - r * nx;
+  const int j = g.ng - (f == 1) + r;
   const int kk = g.ng - (f == 2) + blockIdx.z;
-  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || kk >= g.ngk - g.ng) return;
+  if (j >= g.ngj - g.ng || kk >= g.ngk - g.ng) return;
   const long long c = fst_idx(g, i, j, kk);
   const fst64::Fused k(P.nv);
   if (f == 0) face_terms3d<0>(g, P, k, c, U, rho, vel, Y, red, S, MF);
@@ -235,10 +241,11 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
                                                 double* __restrict__ Rout,
                                                 const double* __restrict__ met, int roles) {
   const int role = blockIdx.x % roles;
-  const int i = g.ng + blockIdx.x / roles * blockDim.x + threadIdx.x;
-  const int j = g.ng + blockIdx.y * blockDim.y + threadIdx.y;
+  const int t = blockIdx.x / roles * 128 + threadIdx.x, r = t / g.nci;  // row after row
+  const int i = g.ng + t - r * g.nci;
+  const int j = g.ng + r;
   const int kk = g.ng + blockIdx.z;
-  if (i >= g.ngi - g.ng || j >= g.ngj - g.ng || kk >= g.ngk - g.ng) return;
+  if (j >= g.ngj - g.ng) return;
   const long long c = fst_idx(g, i, j, kk);
   const long long sv = g.sv, sx = 1, sy = g.sy, sz = g.sz;
   const int nv = P.nv;
@@ -421,17 +428,16 @@ int fst_plain3d_stage(const Geo& g, const Phys& P, const Plain3DBufs& b, const d
                                                        P.visc ? b.Y : nullptr,
                                                        P.ceq ? b.nrg : nullptr, nullptr,
                                                        P.ceq ? b.red : nullptr, b.met));
-  const dim3 bf(32, 4, 1);
-  const dim3 gf(cdiv(g.nci + 1, 32), cdiv(g.ncj + 1, 4), g.nck + 1);
   FST_LAUNCH(prof, "flux3d", st, n, fstflux::launch<true>(g, P, 3, Uin, b.pr, b.vel, b.F, st));
   if (P.visc || P.ceq) {
+    const dim3 gf(3 * cdiv((long long)(g.nci + 1) * (g.ncj + 1), 128), 1, g.nck + 1);
     FST_LAUNCH(prof, "faces3d", st, n,
-               k_faces3d<<<dim3(3 * gf.x, gf.y, gf.z), bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.Y, b.red, b.S, b.MF));
+               k_faces3d<<<gf, 128, 0, st>>>(g, P, Uin, b.rho, b.vel, b.Y, b.red, b.S, b.MF));
   }
   const int roles = P.ceq ? 3 : 2;
-  const dim3 gc(cdiv(g.nci, 32) * roles, cdiv(g.ncj, 4), g.nck);
+  const dim3 gc(roles * cdiv((long long)g.nci * g.ncj, 128), 1, g.nck);
   FST_LAUNCH(prof, "cell3d", st, n,
-             k_cell3d<<<gc, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.MF,
+             k_cell3d<<<gc, 128, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.MF,
                                          b.red, Uold, Unew, coef, Rout, b.met, roles));
   if (ghosts && !Rout)
     FST_LAUNCH(prof, "ghost3d", st, n,
