@@ -21,11 +21,16 @@
 // three times and the momenta/energy of U_new twice.
 //
 // Face kernels: blocks of 32x8 threads march along k (up to 16 planes).  Thread
-// (tx, ty) owns column (i0-1+tx, j0-1+ty); it computes the face at i+1/2
-// from the x-stencil, the face at j+1/2 from the y-stencil and, for the
-// 31x7 interior columns, the face at k+1/2; the left x face comes from
-// lane-1 by shuffle, the lower y face through shared memory, the back z face
-// from the previous plane in registers, so every face is computed once.
+// (tx, ty) owns column (i0+tx, j0-1+ty); it computes the face at i+1/2 from the
+// x-stencil, the face at j+1/2 from the y-stencil and the face at k+1/2; row 0
+// takes y faces only, and with its free x share the seven x faces of the block's
+// left edge.  The left x face comes from lane-1 by shuffle (lane 0: through shared
+// memory), the lower y face through shared memory, the back z face from the previous
+// plane in registers, so a block computes every face once: 32x7 columns.  (31x7
+// columns, with lane 0 left for the edge, put a fifth more blocks on rows that are
+// multiples of 32; per launch at 256^3 and 128^3: k_mspec3d with the equation of
+// state 1438 -> 1280 us and 220 -> 176, k_mmom3d 1027 -> 943 and 160 -> 133; where
+// both give as many blocks, at 200x150x100, 183 -> 186 and 187 -> 189.)
 //
 // Plane data come in by TMA: one elected thread issues cp.async.bulk.tensor
 // 4D copies of a 40x13 (x, y) box of consecutive fields -- the columns plus
@@ -73,24 +78,32 @@ constexpr int NRING = 5;                       // velocity planes k-2 .. k+2
 
 __host__ __device__ constexpr int al32(int n) { return (n + 31) & ~31; }  // 128-byte multiples
 
-// Face-kernel placement: thread (tx, ty) owns column i = ng-1 + 31 bx + tx
-// and row j = ng-1 + 7 by + ty.  The tile starts at x0 = (i_lane0 - 2)
-// rounded down to a multiple of 4 (a TMA box must start on a 16-byte
-// boundary) and at y0 = j_row0 - 2; with ng = 3 both are >= 0.  own: the
-// thread's cell in the tile; its stencils span columns own-2 .. own+3
-// (<= 39) and rows -2 .. +3 (<= 12).
+// Face-kernel placement: thread (tx, ty) owns column i = ng + 32 bx + tx and row
+// j = ng-1 + 7 by + ty.  The tile starts at x0 = i_lane0 - 3 rounded down to a
+// multiple of 4 (a TMA box must start on a 16-byte boundary; with ng = 3 it is one)
+// and at y0 = j_row0 - 2; both are >= 0.  own: the thread's cell in the tile.  Row 0
+// is the row below the block's cells and has only y faces to compute; its lanes 1..7
+// take the x faces at the block's left edge, row `lane` each: xown, (xi, xj) is the
+// cell left of the x face a thread computes, its own in the other rows.  Stencils
+// span columns -2 .. +3 of these (0 <= .. <= 37) and rows -2 .. +3 (<= 12).
 struct Place {
   int i, j, x0, y0, own;
+  int xi, xj, xown;
 };
 __device__ __forceinline__ Place place_faces(const Geo& g) {
   Place p;
-  const int ib = g.ng - 1 + (TX - 1) * (int)blockIdx.x;
+  const int tx = (int)threadIdx.x, ty = (int)threadIdx.y;
+  const int ib = g.ng + TX * (int)blockIdx.x;
   const int jb = g.ng - 1 + (TY - 1) * (int)blockIdx.y;
-  p.i = ib + (int)threadIdx.x;
-  p.j = jb + (int)threadIdx.y;
-  p.x0 = (ib - 2) & ~3;
+  p.i = ib + tx;
+  p.j = jb + ty;
+  p.x0 = (ib - 3) & ~3;
   p.y0 = jb - 2;
   p.own = (p.j - p.y0) * HX + (p.i - p.x0);
+  const bool edge = ty == 0 && tx < TY;  // lane 0 computes none
+  p.xi = edge ? ib - 1 : p.i;
+  p.xj = edge ? jb + tx : p.j;
+  p.xown = (p.xj - p.y0) * HX + (p.xi - p.x0);
   return p;
 }
 // Cell-kernel placement: 32x8 interior cells per block, i = ng + 32 bx + tx;
@@ -104,6 +117,7 @@ __device__ __forceinline__ Place place_cells(const Geo& g) {
   p.x0 = (ib - 2) & ~3;
   p.y0 = jb - 2;
   p.own = (p.j - p.y0) * HX + (p.i - p.x0);
+  p.xi = p.xj = p.xown = 0;
   return p;
 }
 
@@ -552,10 +566,12 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
   const int i = pl.i, j = pl.j;
   const int kc0 = g.ng + (int)blockIdx.z * kz;
   const int kc1 = min(kc0 + kz, g.ngk - g.ng);
-  const bool fi = i <= g.ngi - g.ng - 1;
-  const bool fj = j <= g.ngj - g.ng - 1;
-  const bool ci = tx >= 1 && i >= g.ng && i < g.ngi - g.ng;
-  const bool cj = ty >= 1 && j >= g.ng && j < g.ngj - g.ng;
+  const bool ci = i < g.ngi - g.ng;
+  const bool cj = ty >= 1 && j < g.ngj - g.ng;
+  const bool fj = j < g.ngj - g.ng;
+  // this thread's x face: its cell's upper one, or in row 0 the left edge of row tx
+  const bool fx = (ty >= 1 ? ci : tx >= 1 && tx < TY) && pl.xj < g.ngj - g.ng;
+  const long long cqx0 = (long long)pl.xi + gq.sy * pl.xj;
   const bool cell_col = ci && cj;
   const bool in_arr = i < g.ngi && j < g.ngj;
   const long long cq0 = (long long)i + gq.sy * j;
@@ -637,15 +653,15 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
     const float* tb = tiles + b * L.size;
     const long long cqk = cq0 + gq.sz * k;
     float* sGk = sG + (n & 1) * (TY * TX * NS);
-    if (ok && fi && cj) {  // x face at i+1/2
-      const float* tv = tb + L.v + pl.own;
+    if (ok && fx) {  // x face
+      const float* tv = tb + L.v + pl.xown;
       const float uf = face_u(tv[-1], tv[0], tv[1], tv[2]);
       const bool neg = uf < 0.0f;
-      const bool sm = HYB && smooth_at(smap, cqk, 0);
+      const bool sm = HYB && smooth_at(smap, cqx0 + gq.sz * k, 0);
       const float sc = uf * rd0;
 #pragma unroll
       for (int s = 0; s < NS; ++s)
-        Gx[s] = sc * rec5<HYB>(tb + L.q + s * PL + pl.own, neg ? 3 : -2, neg ? -1 : 1, sm);
+        Gx[s] = sc * rec5<HYB>(tb + L.q + s * PL + pl.xown, neg ? 3 : -2, neg ? -1 : 1, sm);
     }
     if (ok && fj && ci) {  // y face at j+1/2
       const float* tv = tb + L.v + PL + pl.own;
@@ -659,7 +675,10 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
                                neg ? -HX : HX, sm);
     }
 #pragma unroll
-    for (int s = 0; s < NS; ++s) sGk[(ty * TX + tx) * NS + s] = Gy[s];
+    for (int s = 0; s < NS; ++s) {  // the last row's y faces are its own; the edge's x faces take their place
+      if (ty < TY - 1) sGk[(ty * TX + tx) * NS + s] = Gy[s];
+      if (ty == 0 && tx < TY) sGk[((TY - 1) * TX + tx) * NS + s] = Gx[s];
+    }
     if (!__syncthreads_and(ok)) {
       ok = false;
       break;
@@ -680,7 +699,8 @@ __global__ void __launch_bounds__(TX * TY, EPI ? 2 : 3)
     float R[NS];
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const float gxl = __shfl_up_sync(0xffffffffu, Gx[s], 1);
+      float gxl = __shfl_up_sync(0xffffffffu, Gx[s], 1);
+      if (tx == 0) gxl = sGk[((TY - 1) * TX + ty) * NS + s];
       R[s] = 0.f;
       if (cell_col)
         R[s] = -((Gx[s] - gxl) + (Gy[s] - sGk[((ty - 1) * TX + tx) * NS + s]) + (Gzn[s] - Gz[s]));
@@ -807,14 +827,17 @@ __global__ void __launch_bounds__(TX * TY, 2)
   const int i = pl.i, j = pl.j;
   const int kc0 = g.ng + (int)blockIdx.z * kz;
   const int kc1 = min(kc0 + kz, g.ngk - g.ng);
-  const bool fi = i <= g.ngi - g.ng - 1;
-  const bool fj = j <= g.ngj - g.ng - 1;
-  const bool ci = tx >= 1 && i >= g.ng && i < g.ngi - g.ng;
-  const bool cj = ty >= 1 && j >= g.ng && j < g.ngj - g.ng;
+  const bool ci = i < g.ngi - g.ng;
+  const bool cj = ty >= 1 && j < g.ngj - g.ng;
+  const bool fj = j < g.ngj - g.ng;
+  // this thread's x face: its cell's upper one, or in row 0 the left edge of row tx
+  const bool fx = (ty >= 1 ? ci : tx >= 1 && tx < TY) && pl.xj < g.ngj - g.ng;
+  const long long cqx0 = (long long)pl.xi + gq.sy * pl.xj;
   const bool cell_col = ci && cj;
   const bool in_arr = i < g.ngi && j < g.ngj;
   const long long cq0 = (long long)i + gq.sy * j;
   const long long c0 = (long long)i + g.sy * j;
+  const int dxo = pl.xown - pl.own;
   double* Ub = Rout ? Rout : Unew;  // what k_mcell3d wrote
   const double cf = Rout ? 1.0 : coef;
   float maxS;
@@ -928,18 +951,19 @@ __global__ void __launch_bounds__(TX * TY, 2)
     const float *um = vel_at(k - 1), *u0 = vel_at(k), *u1 = vel_at(k + 1);
     const long long cqk = cq0 + gq.sz * k;
     float* sGk = sG + (n & 1) * (TY * TX * 4);
-    if (ok && fi && cj) {  // x face at i+1/2
-      const float uf = face_u(u0[-1], u0[0], u0[1], u0[2]);
+    if (ok && fx) {  // x face
+      const float *xm = um + dxo, *x0 = u0 + dxo, *x1 = u1 + dxo;
+      const float uf = face_u(x0[-1], x0[0], x0[1], x0[2]);
       const bool neg = uf < 0.0f;
-      const bool sm = HYB && smooth_at(smap, cqk, 0);
+      const bool sm = HYB && smooth_at(smap, cqx0 + gq.sz * k, 0);
       const float sc = uf * fc.rd[0];
 #pragma unroll
       for (int v = 0; v < 4; ++v)
-        Gx[v] = sc * rec5<HYB>(tb + L.q + v * PL + pl.own, neg ? 3 : -2, neg ? -1 : 1, sm);
+        Gx[v] = sc * rec5<HYB>(tb + L.q + v * PL + pl.xown, neg ? 3 : -2, neg ? -1 : 1, sm);
       if (visc || ceq) {
         float gr[3][3], uav[3], mu = 0.f, r = 0.f, chat = 0.f, cn[3] = {0.f, 0.f, 0.f};
-        face_grad<0>(um, u0, u1, fc, gr, uav);
-        const int o = pl.own;
+        face_grad<0>(xm, x0, x1, fc, gr, uav);
+        const int o = pl.xown;
         if (visc) mu = 0.5f * (tb[L.mu + o] + tb[L.mu + o + 1]);
         if (ceq) {
           r = 0.5f * (tb[L.rho + o] + tb[L.rho + o + 1]);
@@ -977,7 +1001,10 @@ __global__ void __launch_bounds__(TX * TY, 2)
       }
     }
 #pragma unroll
-    for (int v = 0; v < 4; ++v) sGk[(ty * TX + tx) * 4 + v] = Gy[v];
+    for (int v = 0; v < 4; ++v) {  // as in k_mspec3d
+      if (ty < TY - 1) sGk[(ty * TX + tx) * 4 + v] = Gy[v];
+      if (ty == 0 && tx < TY) sGk[((TY - 1) * TX + tx) * 4 + v] = Gx[v];
+    }
     ok = ok && wait_vel(k + 2);
     ok = ok && wait_tile(n + 1);
     if (!__syncthreads_and(ok)) {
@@ -1016,7 +1043,8 @@ __global__ void __launch_bounds__(TX * TY, 2)
     float R[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
-      const float gxl = __shfl_up_sync(0xffffffffu, Gx[v], 1);
+      float gxl = __shfl_up_sync(0xffffffffu, Gx[v], 1);
+      if (tx == 0) gxl = sGk[((TY - 1) * TX + ty) * 4 + v];
       R[v] = 0.f;
       if (cell_col)
         R[v] = -((Gx[v] - gxl) + (Gy[v] - sGk[((ty - 1) * TX + tx) * 4 + v]) + (Gzn[v] - Gz[v]));
@@ -1081,7 +1109,7 @@ template <int NS, bool HYB>
 int launch_spec(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                 const unsigned char* smooth, const double* Uold, double* Unew, double coef,
                 double* Rout, cudaStream_t st, bool fused) {
-  const unsigned nx = cdiv3(g.nci, TX - 1), ny = cdiv3(g.ncj, TY - 1);
+  const unsigned nx = cdiv3(g.nci, TX), ny = cdiv3(g.ncj, TY - 1);
   const int kz = plan_kz((long long)nx * ny, g.nck);
   const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = spec_smem(NS);
@@ -1125,7 +1153,7 @@ template <bool HYB>
 void launch_mom(const Geo& g, const Phys& P, const MixedBufs& b, const MixedView& M,
                 const unsigned char* smooth, double* Unew, double coef, double* Rout,
                 cudaStream_t st) {
-  const unsigned nx = cdiv3(g.nci, TX - 1), ny = cdiv3(g.ncj, TY - 1);
+  const unsigned nx = cdiv3(g.nci, TX), ny = cdiv3(g.ncj, TY - 1);
   const int kz = plan_kz((long long)nx * ny, g.nck);
   const dim3 grd(nx, ny, cdiv3(g.nck, kz));
   const size_t sm = mom_smem(P.visc != 0, P.ceq != 0);
