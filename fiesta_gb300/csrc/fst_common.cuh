@@ -39,6 +39,13 @@ struct DivC {
   }
 };
 
+// a/x, b/y, c/z with one call
+__device__ __forceinline__ fst64::Quot3 div3(const DivC& x, double a, const DivC& y, double b, const DivC& z,
+                                             double c) {
+  if (x.k == DivC::NONE && y.k == DivC::NONE && z.k == DivC::NONE) return fst64::div3_call(a, b, c, x.r, y.r, z.r);
+  return {x.call(a), y.call(b), z.call(c)};
+}
+
 // Physics constants of one run, passed by value to the kernels.
 struct Phys {
   int ns, nv, nvt, visc, ceq, buoyancy;

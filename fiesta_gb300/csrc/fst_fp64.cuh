@@ -385,6 +385,15 @@ __device__ __noinline__ static double mul_call(double a, double b) { return mul_
 __device__ __noinline__ static double div_call(double a, uint32_t hi, uint32_t lo, uint32_t R) {
   return div_by(a, Recip{hi, lo, R});
 }
+// three quotients in one call, side by side (div_exact)
+struct Quot3 {
+  double x, y, z;
+};
+__device__ __noinline__ static Quot3 div3_call(double a, double b, double c, Recip ra, Recip rb, Recip rc) {
+  const Quot3 q{div_core(a, ra), div_core(b, rb), div_core(c, rc)};
+  if (div_exact(a, ra) & div_exact(b, rb) & div_exact(c, rc)) return q;
+  return {div_by(a, ra), div_by(b, rb), div_by(c, rc)};
+}
 #endif
 
 }  // namespace fst64

@@ -226,7 +226,11 @@ __global__ void __launch_bounds__(128, 7) k_faces3d(Geo g, Phys P, const double*
 // The variables that share nothing run in different blocks (blockIdx.x % roles):
 // the momenta and energy, the species (advection only), the C variables; loops
 // over the directions stay rolled.  Both keep the code of a block small and give
-// a small grid three times the warps.
+// a small grid three times the warps.  Quotients go three to a call (div3), which
+// shortens the chain that bounds small grids and the calls of all: 256^3, 5 species,
+// 8.31 -> 7.85 ms, 64^3 157 -> 143 us, 21x19x23, 2 species, 33 -> 25 us.  (The same in
+// k_faces3d and k_cell2d costs registers: 6.70 -> 7.22 ms at 256^3, 50 -> 55 us at
+// 400x300.  A block per variable: 27 us at 21x19x23, but 8.97 ms at 256^3.)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* __restrict__ U,
                                                 const double* __restrict__ rho,
@@ -284,10 +288,9 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
     for (int f = 0; f < 3; ++f) {
       const long long s = stride(f);
       const DivC& d12 = P.d12[f];
-      auto d4 = [&](const double* a) {
-        return d12.call(d4sum(a[c - 2 * s], a[c - s], a[c + s], a[c + 2 * s]));
-      };
-      const double r = d4(rho), e = d4(nrg), u = d4(vel + sv * f);
+      auto d4 = [&](const double* a) { return d4sum(a[c - 2 * s], a[c - s], a[c + s], a[c + 2 * s]); };
+      const fst64::Quot3 d = div3(d12, d4(rho), d12, d4(nrg), d12, d4(vel + sv * f));
+      const double r = d.x, e = d.y, u = d.z;
       divu = f == 0 ? u : k.add(divu, u);
       if (f == 0) { gr[0] = r; ge[0] = e; }
       else if (f == 1) { gr[1] = r; ge[1] = e; }
@@ -310,10 +313,10 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
       else Gn = n == 2 ? gr[0] : n == 3 ? gr[1] : gr[2];
       const double* Cn = U + sv * (nv + n);
       const double cc = Cn[c], c2 = twice(cc);
-      const double lx = P.dd[0].call(k.add(k.sub(Cn[c - sx], c2), Cn[c + sx]));
-      const double ly = P.dd[1].call(k.add(k.sub(Cn[c - sy], c2), Cn[c + sy]));
-      const double lz = P.dd[2].call(k.add(k.sub(Cn[c - sz], c2), Cn[c + sz]));
-      const double lap = k.add(k.add(lx, ly), lz);
+      const fst64::Quot3 l = div3(P.dd[0], k.add(k.sub(Cn[c - sx], c2), Cn[c + sx]),  //
+                                  P.dd[1], k.add(k.sub(Cn[c - sy], c2), Cn[c + sy]),
+                                  P.dd[2], k.add(k.sub(Cn[c - sz], c2), Cn[c + sz]));
+      const double lap = k.add(k.add(l.x, l.y), l.z);
       emit(nv + n, k.add(mul_call(src, k.sub(Gn, cc)), mul_call(dif, lap)));
     }
     return;
@@ -364,11 +367,13 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
       const long long s = stride(f);
       const DivC& dd = P.dd[f];
       const double* Sf = S + (long long)f * 6 * sv + c;
-      auto diff = [&](int q) { return dd.call(k.sub(Sf[q * sv], Sf[q * sv - s])); };
-      R0 = k.add(R0, diff(0));
-      R1 = k.add(R1, diff(1));
-      R2 = k.add(R2, diff(2));
-      R3 = k.add(R3, k.add(k.add(diff(3), diff(4)), diff(5)));
+      auto diff = [&](int q) { return k.sub(Sf[q * sv], Sf[q * sv - s]); };
+      const fst64::Quot3 m = div3(dd, diff(0), dd, diff(1), dd, diff(2));
+      R0 = k.add(R0, m.x);
+      R1 = k.add(R1, m.y);
+      R2 = k.add(R2, m.z);
+      const fst64::Quot3 e = div3(dd, diff(3), dd, diff(4), dd, diff(5));
+      R3 = k.add(R3, k.add(k.add(e.x, e.y), e.z));
     }
   }
   if (P.ceq) {  // applyCeq
@@ -380,9 +385,11 @@ __global__ void __launch_bounds__(128, 8) k_cell3d(Geo g, Phys P, const double* 
 #pragma unroll 1
       for (int d = 0; d < 3; ++d) {
         const double* m = MF + (long long)((f * 3 + d) * 3) * sv + c;
-#pragma unroll
-        for (int w = 0; w < 3; ++w)
-          diffu[w] = k.add(diffu[w], dd.call(k.sub(m[w * sv], m[w * sv - s])));
+        auto diff = [&](int w) { return k.sub(m[w * sv], m[w * sv - s]); };
+        const fst64::Quot3 q = div3(dd, diff(0), dd, diff(1), dd, diff(2));
+        diffu[0] = k.add(diffu[0], q.x);
+        diffu[1] = k.add(diffu[1], q.y);
+        diffu[2] = k.add(diffu[2], q.z);
       }
     }
     R0 = k.add(R0, diffu[0]);
