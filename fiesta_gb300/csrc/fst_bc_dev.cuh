@@ -160,7 +160,7 @@ __device__ __forceinline__ GhostSource ghost_source(const Geo& g, const GhostRul
     }
     const int layer = side ? x - (g.ng + n) : g.ng - 1 - x;
     x = side ? g.ng + n - 1 - layer : g.ng + layer;
-    const int t = r.type[a][side];
+    const int t = side ? r.type[a][1] : r.type[a][0];  // (indexed, the rule is copied to local memory)
     q.flip ^= t == FST_BC_NOSLIP ? 7u : t == FST_BC_OUTFLOW ? 0u : 1u << a;
     if (t == FST_BC_HYDROSTATIC) {
       q.layer = layer;

@@ -172,29 +172,34 @@ __host__ __device__ __forceinline__ long long fst_shell_count(const Geo& g) {
   const long long nk = g.ngk - 2 * ngz, nj = g.ngj - 2 * g.ng;
   return 2LL * ngz * g.ngi * g.ngj + nk * 2 * g.ng * g.ngi + nk * nj * 2 * g.ng;
 }
-__device__ __forceinline__ void fst_shell_cell(const Geo& g, long long t, int& i, int& j,
-                                               int& k) {
+template <class T>
+__device__ __forceinline__ void fst_shell_cell_of(const Geo& g, T t, int& i, int& j, int& k) {
   const int ng = g.ng, ngz = g.ndim == 3 ? g.ng : 0;
   const int nj = g.ngj - 2 * ng, nk = g.ngk - 2 * ngz;
-  const long long pl = (long long)g.ngi * g.ngj;
-  const long long nA = 2LL * ngz * pl, nB = (long long)nk * 2 * ng * g.ngi;
+  const T ni = (T)g.ngi, pl = ni * (T)g.ngj, w = (T)(2 * ng);
+  const T nA = 2 * (T)ngz * pl, nB = (T)nk * w * ni;
   if (t < nA) {
-    const long long p = t / pl, r = t - p * pl;
-    k = p < ngz ? (int)p : g.ngk - 2 * ngz + (int)p;
-    j = (int)(r / g.ngi);
-    i = (int)(r - (long long)j * g.ngi);
+    const T p = t / pl, r = t - p * pl;
+    k = (int)p < ngz ? (int)p : g.ngk - 2 * ngz + (int)p;
+    j = (int)(r / ni);
+    i = (int)(r - (T)j * ni);
   } else if (t < nA + nB) {
-    const long long u = t - nA, row = u / g.ngi;
-    i = (int)(u - row * g.ngi);
-    const int kk = (int)(row / (2 * ng)), jj = (int)(row - (long long)kk * 2 * ng);
+    const T u = t - nA, row = u / ni;
+    i = (int)(u - row * ni);
+    const int kk = (int)(row / w), jj = (int)(row - (T)kk * w);
     k = ngz + kk;
     j = jj < ng ? jj : g.ngj - 2 * ng + jj;
   } else {
-    const long long u = t - nA - nB, row = u / (2 * ng);
-    const int ii = (int)(u - row * 2 * ng);
-    const int kk = (int)(row / nj), jj = (int)(row - (long long)kk * nj);
+    const T u = t - nA - nB, row = u / w;
+    const int ii = (int)(u - row * w);
+    const int kk = (int)(row / (T)nj), jj = (int)(row - (T)kk * (T)nj);
     k = ngz + kk;
     j = ng + jj;
     i = ii < ng ? ii : g.ngi - 2 * ng + ii;
   }
+}
+// (64-bit divisions are most of the instructions of a ghost cell: only where needed)
+__device__ __forceinline__ void fst_shell_cell(const Geo& g, long long t, int& i, int& j, int& k) {
+  if (g.sv <= 0x7FFFFFFFLL) fst_shell_cell_of(g, (unsigned)t, i, j, k);
+  else fst_shell_cell_of(g, t, i, j, k);
 }
