@@ -228,10 +228,10 @@ def algorithmic_bytes(kernel, cfg):
 # not run inside the bench, so these are the captured figures, labelled so in
 # the line.
 TRAFFIC_BYTES_PER_LAUNCH_256 = {
-    "mspec3d_eos": 4.078e9,
-    "mmom3d": 1.936e9,
-    "mceq3d": 2.807e9,
-    "mcell3d": 1.167e9,
+    "mspec3d_eos": 4.074e9,
+    "mmom3d": 1.950e9,
+    "mceq3d": 2.814e9,
+    "mcell3d": 1.165e9,
 }
 
 
@@ -323,8 +323,8 @@ def run_gpu_mode(mode_name, n, steps, warmup, U0, dt, peak_gbs, peak_kind, e2e_s
             from fiesta_gb300.solver import fp64_rate
             roof["fp64_peak_gflops_measured"] = fp64_rate(stream.cuda_stream)
             roof["bound"] = "fp64"
-            roof["bound_note"] = ("FP64 pipe 85 % busy, DRAM a few % (an ncu capture of "
-                                  "k_flux3d at 64^3); the GB/s figures show how far below the "
+            roof["bound_note"] = ("FP64 pipe 82 % busy, DRAM a few % (an ncu capture of "
+                                  "k_weno_flux at 128^3); the GB/s figures show how far below the "
                                   "HBM roof an FP64-bound kernel sits")
 
     # end to end through the C ABI with host buffers: upload, step, download.
