@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(128) k_faces2d(Geo g, Phys P, const double* __
 // applyViscousTerm2dv, calculateRhoGrad2D, updateCeq2D, applyCeq2D, then the
 // stage combine (src/rk.cpp:42-69).  blockIdx.z: 0 the momenta and energy, 1 the
 // species, 2 the C variables, which share nothing.
-__global__ void __launch_bounds__(128) k_cell2d(Geo g, Phys P, const double* __restrict__ U,
+template <int PER_SM>
+__global__ void __launch_bounds__(128, PER_SM) k_cell2d(Geo g, Phys P, const double* __restrict__ U,
                                                 const double* __restrict__ rho,
                                                 const double* __restrict__ pr,
                                                 const double* __restrict__ vel,
@@ -424,9 +425,15 @@ int fst_plain2d_stage(const Geo& g, const Phys& P, const Plain2DBufs& b, const d
                k_faces2d<<<dim3(gf.x, gf.y, 2), bf, 0, st>>>(g, P, Uin, b.rho, b.vel, b.T, b.red, b.S, b.Q, b.MF));
   }
   const dim3 gc(cdiv(g.nci, 32), cdiv(g.ncj, 4), P.ceq ? 3 : 2);
+  // Blocks per SM: what 72 registers a thread give (7; no bound set) while the launch is
+  // a few waves long and a thread's chain counts, 10 (48 registers, some spilled) where
+  // the FP64 unit's share does.  72 registers against 48: 200x100 15.4 and 16.2 us,
+  // 400x300 (2925 blocks) 49.9 and 50.8, 600x500 (7125) 126 and 116, 999^2 369 and 328;
+  // 12 blocks: 320 there, but 53 at 400x300.
+  auto cell = gc.x * gc.y * gc.z > 4 * 7 * 152 ? k_cell2d<10> : k_cell2d<0>;
   FST_LAUNCH(prof, "cell2d", st, n,
-             k_cell2d<<<gc, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.Q,
-                                         b.MF, b.red, Uold, Unew, coef, Rout, b.met));
+             cell<<<gc, bf, 0, st>>>(g, P, Uin, b.rho, b.pr, b.vel, b.nrg, b.F, b.S, b.Q,
+                                     b.MF, b.red, Uold, Unew, coef, Rout, b.met));
   if (ghosts && !Rout) {
     FST_LAUNCH(prof, "ghost2d", st, n,
                k_ghost2d<<<cdiv(g.sv, 256), 256, 0, st>>>(g, Uold, Unew, coef));
