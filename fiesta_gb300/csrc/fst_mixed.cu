@@ -12,7 +12,7 @@
 //
 // Per stage: k_mprim over all cells (FP64 state -> FP32 primitives + FP64
 // p, and the C-equation maxima maxS, maxCh by block max + atomicMax), then
-// the fused right-hand side + RK stage: in 3D the two TMA-fed kernels of
+// the fused right-hand side + RK stage: in 3D the TMA-fed kernels of
 // fst_mixed3d.cu, in 2D k_mrhs2d below (a 32x8 tile of columns; each thread
 // computes the faces at i+1/2 and j+1/2 once, the left x face by shuffle,
 // the lower y face through shared memory; every face carries nv FP32

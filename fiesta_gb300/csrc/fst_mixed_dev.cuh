@@ -9,7 +9,6 @@ namespace fstm {
 
 constexpr int TX = 32;  // tile width (threads along i)
 constexpr int TY = 8;   // tile height (threads along j)
-constexpr int KZ = 16;  // planes per block along k
 constexpr int NVMAX = 4 + FST_MAX_SPECIES;
 
 // ---------------------------------------------------------------------------
