@@ -38,11 +38,15 @@ __device__ __forceinline__ int find_case(const int* __restrict__ off, int n, int
 // persistent RHS + RK stage over the (case, tile) work list: block b takes
 // work items b, b + gridDim.x, ...; item w is tile w - tile_off[c] of case c
 // (tiles of a case in row-major order, (nci + TXX - 2) / (TXX - 1) per row).
-// Bound by the latency of the tile's gathers.  1280 threads per SM (48 registers):
-// the 24-case, 1.5 M cell step takes 543 us, 554 at 1024 threads, 703 with the
-// registers the two faces' loads would take (768 threads).
+// Bound by the latency of the tile's gathers: warps in flight matter more than the
+// registers the two faces' loads would take.  1280 threads per SM (1024 where a block
+// has 512): 48 registers, at 4 to 8 variables up to 140 bytes a thread spilled.  Step of
+// the 24-case, 1.5 M cell ensemble, one gas, two, ... six, viscous with C-equation, in
+// us: one face after the other 509, 580, 629, 722, 779, 1523; both at once and no bound
+// 670, 713, 759, 955, 1030, 1445; at 768 threads 590, 625, 665, 751, 803, 1224; at 1024
+// 525, 557, 589, 676, 739, 1124; at 1280 513, 540, 582, 682, 736, 1098.
 template <int NV, int TYY, int TXX>
-__global__ void __launch_bounds__(TXX * TYY, NV <= 8 ? 1280 / (TXX * TYY) : 1) k_brhs(const BCase* __restrict__ cs,
+__global__ void __launch_bounds__(TXX * TYY, 1280 / (TXX * TYY)) k_brhs(const BCase* __restrict__ cs,
                                                     const Phys* __restrict__ Ps,
                                                     const int* __restrict__ tile_off, int ncase,
                                                     int stage) {

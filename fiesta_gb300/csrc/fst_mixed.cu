@@ -188,8 +188,14 @@ __global__ void __launch_bounds__(256) k_mupload3(Geo g, Geo gq, Phys P,
   if (red) block_max_256(red, lS, lC);
 }
 
+// The 2D tile on a single case.  4 blocks per SM (64 registers): both faces' loads would
+// take up to 123 and leave 3 or 2 blocks.  Step at 900^2, viscous with C-equation, in us,
+// with 1, 2, 4, 6 and 8 gases: no bound 272, 302, 409, 519, 753; 3 blocks 301, 323, 383,
+// 465, 647; 4 blocks 260, 287, 351, 437, 598; 5 blocks 255, 289, 360, 458, 584, but at
+// 300^2 they lose 2 to 10 % to 4.  Learned routing with 5 and 6 gases: no bound 645, 687,
+// 4 blocks 471, 539.  One face after the other, no bound: 260, 303, 373, 466, 817; 510, 526.
 template <int NV, bool HYB>
-__global__ void __launch_bounds__(TX * TY) k_mrhs2d(Geo g, Phys P, MixedView M,
+__global__ void __launch_bounds__(TX * TY, 4) k_mrhs2d(Geo g, Phys P, MixedView M,
                                                     const unsigned long long* __restrict__ red,
                                                     const unsigned char* __restrict__ smap,
                                                     const double* Uold, double* Unew, double coef,
