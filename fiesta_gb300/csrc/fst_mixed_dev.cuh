@@ -110,12 +110,12 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
   auto species = [&](int s) { return NS > 0 ? us[s] : U[c + sv * (s0 + s)]; };
   auto momentum = [&](int d) { return NS > 0 ? um[d] : U[c + sv * d]; };  // NDIM: the energy
   const int ns = NS > 0 ? NS : P.ns;
+  // (a loop over any number of species is left to the compiler: unrolled 16 times with an
+  // exit per species the pass of the 24-case ensemble takes 239 us against 164 with 6 gases)
   // mixture EOS (calculateRhoPT, src/secondary.hpp:60-151)
   double sCv = 0.0, sRm = 0.0, r64 = 0.0;
   float rf = 0.f;
-#pragma unroll
-  for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
-    if (NS == 0 && s >= ns) break;
+  for (int s = 0; s < ns; ++s) {
     const double rs = species(s);
     if (rho64) r64 += rs;
     sCv = fma(rs, P.cv_s[s], sCv);
@@ -125,9 +125,7 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
   const float rif = __frcp_rn(rf);
   const double gm1 = sRm * rcp64(sCv);
   float Cv2 = 0.f, Cp2 = 0.f, m = 0.f;
-#pragma unroll
-  for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
-    if (NS == 0 && s >= ns) break;
+  for (int s = 0; s < ns; ++s) {
     const float rs = d2f(species(s));
     const float ys = rs * rif;
     if (NDIM == 2) {
@@ -166,9 +164,7 @@ __device__ __forceinline__ void mprim_cell(const Geo& g, const Geo& gq, const Ph
     // replace the FP32 values above), for the shock and contact switches;
     // lo = [rho, nrg, u, v] low parts (see Prim3Out)
     f2p r = {0.f, 0.f};
-#pragma unroll
-    for (int s = 0; s < (NS > 0 ? NS : FST_MAX_SPECIES); ++s) {
-      if (NS == 0 && s >= ns) break;
+    for (int s = 0; s < ns; ++s) {
       r = df_add(r, split(species(s)));
     }
     f2p m2 = {0.f, 0.f};

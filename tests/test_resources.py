@@ -45,3 +45,22 @@ def test_2d_tile_keeps_its_warps(tmp_path):
         threads = 256 if single else int(batch.group(2)) * int(batch.group(3))
         assert _resident(regs, threads) >= 1024, (name, regs)
     assert seen == 14 + 48  # 7 variable counts with and without routing; 6 counts, 8 shapes
+
+
+def _primitive_passes(tmp):
+    """[(is k_bprim, species or 0 for any number, registers)] of the 2D primitive passes."""
+    out = []
+    for name, regs in _ptxas("fst_batch.cu", tmp)[0] + _ptxas("fst_mixed.cu", tmp)[0]:
+        m = re.search(r"(k_bprimI|k_mprimILi2E)Li(\d+)E", name)
+        if m:
+            out.append((m.group(1) == "k_bprimI", int(m.group(2)), regs))
+    return out
+
+
+def test_any_species_primitive_pass_keeps_its_warps(tmp_path):
+    """The passes whose species count is not known at compile time: their loops are not
+    unrolled 16 times."""
+    found = [(batch, regs) for batch, ns, regs in _primitive_passes(str(tmp_path)) if ns == 0]
+    assert len(found) == 2
+    for batch, regs in found:
+        assert _resident(regs, 256) >= (768 if batch else 1024), (batch, regs)
