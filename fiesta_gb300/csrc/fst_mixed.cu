@@ -54,8 +54,10 @@ __device__ __forceinline__ void block_max_256(unsigned long long* red, float lS,
   }
 }
 
+// 4 blocks per SM: with the registers that 4 and 5 species would take it is 3, and 51.0 and
+// 55.7 us a launch at 900^2 (C-equation) against 46.3 and 51.6.
 template <int NDIM, int NS>
-__global__ void __launch_bounds__(256) k_mprim(Geo g, Geo gq, Phys P, const double* __restrict__ U,
+__global__ void __launch_bounds__(256, 4) k_mprim(Geo g, Geo gq, Phys P, const double* __restrict__ U,
                                                float* __restrict__ Q, float* __restrict__ rho,
                                                double* __restrict__ rho64,
                                                float* __restrict__ vel, double* __restrict__ pr,

@@ -64,3 +64,11 @@ def test_any_species_primitive_pass_keeps_its_warps(tmp_path):
     assert len(found) == 2
     for batch, regs in found:
         assert _resident(regs, 256) >= (768 if batch else 1024), (batch, regs)
+
+
+def test_primitive_passes_keep_their_warps(tmp_path):
+    """The passes of 1 to 5 species."""
+    found = [(batch, ns, regs) for batch, ns, regs in _primitive_passes(str(tmp_path)) if ns > 0]
+    assert len(found) == 10
+    for batch, ns, regs in found:
+        assert _resident(regs, 256) >= (768 if batch else 1024), (batch, ns, regs)
