@@ -119,12 +119,13 @@ __global__ void k_bface(const BCase* __restrict__ cs, int axis, int side, bool u
   fstbc::face_line(g, use_a ? B.Ua : B.Ub, axis, side, B.bc[axis * 2 + side], t, 0);
 }
 
-// primitive pass: block b belongs to case find_case(block_off, b).  3 blocks per SM: with
-// the registers that 4 and 5 species would take it is 2, and 121 and 130 us a launch over
+// primitive pass: block b belongs to case find_case(block_off, b).  3 blocks per SM.  With
+// 4 and 5 species the compiler would take registers for 2, and 121 and 130 us a launch over
 // the 24 cases of 1.5 M cells (C-equation) against 101 and 113; at 4 blocks (64 registers)
-// 100 and 111, but ensembles of a few small cases lose up to a fifth.
+// 100 and 111, but ensembles of a few small cases lose up to a fifth.  Fewer species keep
+// to 80 registers by themselves (a bound makes them spill: step 525 us against 522).
 template <int NS>
-__global__ void __launch_bounds__(256, 3) k_bprim(const BCase* __restrict__ cs,
+__global__ void __launch_bounds__(256, NS > 3 ? 3 : 0) k_bprim(const BCase* __restrict__ cs,
                                                const Phys* __restrict__ Ps,
                                                const int* __restrict__ block_off, int ncase,
                                                int stage, bool red) {
