@@ -39,14 +39,14 @@ __device__ __forceinline__ int find_case(const int* __restrict__ off, int n, int
 // work items b, b + gridDim.x, ...; item w is tile w - tile_off[c] of case c
 // (tiles of a case in row-major order, (nci + TXX - 2) / (TXX - 1) per row).
 // Bound by the latency of the tile's gathers: warps in flight matter more than the
-// registers the two faces' loads would take.  1280 threads per SM (1024 where a block
-// has 512): 48 registers, at 4 to 8 variables up to 140 bytes a thread spilled.  Step of
-// the 24-case, 1.5 M cell ensemble, one gas, two, ... six, viscous with C-equation, in
-// us: one face after the other 509, 580, 629, 722, 779, 1523; both at once and no bound
-// 670, 713, 759, 955, 1030, 1445; at 768 threads 590, 625, 665, 751, 803, 1224; at 1024
-// 525, 557, 589, 676, 739, 1124; at 1280 513, 540, 582, 682, 736, 1098.
+// registers.  1280 threads per SM (1024 where a block has 512): 48 registers, at 5 to 8
+// variables 68 to 96 bytes a thread spilled; 1024 beyond, where 48 registers spill 600.
+// Launch over the 24 cases of 1.5 M cells, C-equation on, one gas, two, ... six, in us: one
+// face after the other and no bound 160, 184, 205, 225, 242, 491; as here 160, 173, 187,
+// 199, 213, 298.  Both faces at once and no bound, a step: 670, 713, 759, 955, 1030, 1445;
+// at 1280 threads 513, 540, 582, 682, 736, 1098.
 template <int NV, int TYY, int TXX>
-__global__ void __launch_bounds__(TXX * TYY, 1280 / (TXX * TYY)) k_brhs(const BCase* __restrict__ cs,
+__global__ void __launch_bounds__(TXX * TYY, (NV <= 8 ? 1280 : 1024) / (TXX * TYY)) k_brhs(const BCase* __restrict__ cs,
                                                     const Phys* __restrict__ Ps,
                                                     const int* __restrict__ tile_off, int ncase,
                                                     int stage) {

@@ -190,14 +190,15 @@ __global__ void __launch_bounds__(256) k_mupload3(Geo g, Geo gq, Phys P,
   if (red) block_max_256(red, lS, lC);
 }
 
-// The 2D tile on a single case.  4 blocks per SM (64 registers): both faces' loads would
-// take up to 123 and leave 3 or 2 blocks.  Step at 900^2, viscous with C-equation, in us,
-// with 1, 2, 4, 6 and 8 gases: no bound 272, 302, 409, 519, 753; 3 blocks 301, 323, 383,
-// 465, 647; 4 blocks 260, 287, 351, 437, 598; 5 blocks 255, 289, 360, 458, 584, but at
-// 300^2 they lose 2 to 10 % to 4.  Learned routing with 5 and 6 gases: no bound 645, 687,
-// 4 blocks 471, 539.  One face after the other, no bound: 260, 303, 373, 466, 817; 510, 526.
-template <int NV, bool HYB>
-__global__ void __launch_bounds__(TX * TY, 4) k_mrhs2d(Geo g, Phys P, MixedView M,
+// The 2D tile on a single case.  4 blocks per SM (64 registers): left alone the compiler
+// takes up to 123 and leaves 3 or 2 blocks.  Step at 900^2, viscous with C-equation, in us,
+// with 1, 2, 4 and 6 gases: no bound 260 (one face after the other; 272 both at once), 303
+// (302), 373 (409), 466 (519); 3 blocks 301, 323, 404, 481; 4 blocks 260, 287, 355, 432; 5
+// blocks 255, 289, 348, 412, but at 300^2 they lose up to 11 %.  More than 9 variables spill
+// at 64 registers; a grid that two blocks per SM hold at once has no use for more, and takes
+// the registers instead (9 gases, 64x48: 16.4 us against 17.8; 300^2 28.6 against 19.8).
+template <int NV, bool HYB, int PER_SM>
+__global__ void __launch_bounds__(TX * TY, PER_SM) k_mrhs2d(Geo g, Phys P, MixedView M,
                                                     const unsigned long long* __restrict__ red,
                                                     const unsigned char* __restrict__ smap,
                                                     const double* Uold, double* Unew, double coef,
@@ -299,7 +300,11 @@ void launch_rhs(const Geo& g, const Phys& P, const MixedView& M, const unsigned 
                 double* Rout, cudaStream_t st) {
   const dim3 blk(TX, TY, 1);
   const dim3 grd(cdiv(g.nci, TX - 1), cdiv(g.ncj, TY - 1), 1);
-  k_mrhs2d<NV, HYB><<<grd, blk, 0, st>>>(g, P, M, red, smap, Uold, Unew, coef, Rout);
+  auto run = [&](auto kernel) {
+    kernel<<<grd, blk, 0, st>>>(g, P, M, red, smap, Uold, Unew, coef, Rout);
+  };
+  if (NV == NVMAX && grd.x * grd.y <= 2 * 152) run(k_mrhs2d<NV, HYB, NV == NVMAX ? 2 : 4>);
+  else run(k_mrhs2d<NV, HYB, 4>);
 }
 
 template <bool HYB>

@@ -426,13 +426,33 @@ __device__ __forceinline__ bool smooth_at(const unsigned char* map, long long c,
 // 2D face terms of cart2d (src/flux.hpp:23-106, src/viscosity.hpp:25-199,
 // src/ceq.hpp:200-293) with their quirks, in FP32.
 // ---------------------------------------------------------------------------
-// WENO fluxes of the faces at (cx + 1/2, .) and (., cy + 1/2), both at once and
-// without a branch, so that the loads of one are in flight while the other's are
-// used (a face out of range is given a clamped cell and dropped by the caller).
+// WENO fluxes of the upper face of cell c along f.
 template <int NV, bool HYB>
+__device__ __forceinline__ void face2d_weno(const Geo& g, const MixedView& M, const FaceCtx& fc,
+                                            long long c, int f, bool smooth, int nv, float* G) {
+  const long long sv = g.sv, sf = f == 0 ? 1 : g.sy;
+  const float* un = M.vel + sv * f;
+  const float uf = (-un[c + 2 * sf] + 7.0f * un[c + sf] + 7.0f * un[c] - un[c - sf]) * (1.0f / 12.0f);
+  const bool neg = uf < 0.0f;
+  const long long c0 = neg ? c + 3 * sf : c - 2 * sf;
+  const long long o = neg ? -sf : sf;
+  const float scale = uf * fc.rd[f];
+#pragma unroll
+  for (int w = 0; w < NV; ++w) {
+    if (NV == NVMAX && w >= nv) break;
+    const float* q = M.Q + sv * w;
+    const float f1 = __ldg(q + c0), f2 = __ldg(q + c0 + o), f3 = __ldg(q + c0 + 2 * o),
+                f4 = __ldg(q + c0 + 3 * o), f5 = __ldg(q + c0 + 4 * o);
+    G[w] = scale * ((HYB && smooth) ? upwind5_f(f1, f2, f3, f4, f5) : weno_f(f1, f2, f3, f4, f5));
+  }
+}
+
+// The same of the x and the y face of cell c, both at once and without a branch, so
+// that the loads of one are in flight while the other's are used (a face out of range
+// is given a clamped cell and dropped by the caller).
+template <int NV>
 __device__ __forceinline__ void faces2d_weno(const Geo& g, const MixedView& M, const FaceCtx& fc,
-                                             long long c, bool smx, bool smy, int nv, float* Gx,
-                                             float* Gy) {
+                                             long long c, float* Gx, float* Gy) {
   const long long sv = g.sv, sy = g.sy;
   const float* u = M.vel;
   const float* v = M.vel + sv;
@@ -443,14 +463,13 @@ __device__ __forceinline__ void faces2d_weno(const Geo& g, const MixedView& M, c
   const float sx_ = ux * fc.rd[0], sy_ = uy * fc.rd[1];
 #pragma unroll
   for (int w = 0; w < NV; ++w) {
-    if (NV == NVMAX && w >= nv) break;
     const float* q = M.Q + sv * w;
     const float a1 = __ldg(q + cx), a2 = __ldg(q + cx + ox), a3 = __ldg(q + cx + 2 * ox),
                 a4 = __ldg(q + cx + 3 * ox), a5 = __ldg(q + cx + 4 * ox);
     const float b1 = __ldg(q + cy), b2 = __ldg(q + cy + oy), b3 = __ldg(q + cy + 2 * oy),
                 b4 = __ldg(q + cy + 3 * oy), b5 = __ldg(q + cy + 4 * oy);
-    Gx[w] = sx_ * ((HYB && smx) ? upwind5_f(a1, a2, a3, a4, a5) : weno_f(a1, a2, a3, a4, a5));
-    Gy[w] = sy_ * ((HYB && smy) ? upwind5_f(b1, b2, b3, b4, b5) : weno_f(b1, b2, b3, b4, b5));
+    Gx[w] = sx_ * weno_f(a1, a2, a3, a4, a5);
+    Gy[w] = sy_ * weno_f(b1, b2, b3, b4, b5);
   }
 }
 
@@ -548,15 +567,29 @@ __device__ __forceinline__ void rhs2d_tile(const Geo& g, const Phys& P, const Mi
 #pragma unroll
   for (int v = 0; v < NV; ++v) Gx[v] = Gy[v] = 0.f;
   const bool vx = fi && cj, vy = fj && ci;
-  const long long cf = (long long)min(i, g.ngi - g.ng - 1) + sy * min(j, g.ngj - g.ng - 1);
-  faces2d_weno<NV, HYB>(g, M, fc, cf, HYB && smooth_at(smap, cf, 0), HYB && smooth_at(smap, cf, 1),
-                        nv, Gx, Gy);
-  face2d_terms(g, P, M, fc, cf, 0, Gx);
-  face2d_terms(g, P, M, fc, cf, 1, Gy);
+  // Both faces at once up to 6 variables and without routing.  Beyond, their registers
+  // spill at 4 blocks per SM and the overlap no longer pays: k_mrhs2d at 300^2, 9 variables,
+  // 13.8 us against 11.8, with routing 14.2 against 12.2; a step at 900^2 with 8 variables
+  // and routing 471 us against 453, with 9 540 against 511.
+  if constexpr (NV <= 6 && !HYB) {
+    const long long cf = (long long)min(i, g.ngi - g.ng - 1) + sy * min(j, g.ngj - g.ng - 1);
+    faces2d_weno<NV>(g, M, fc, cf, Gx, Gy);
+    face2d_terms(g, P, M, fc, cf, 0, Gx);
+    face2d_terms(g, P, M, fc, cf, 1, Gy);
 #pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    Gx[v] = vx ? Gx[v] : 0.f;
-    Gy[v] = vy ? Gy[v] : 0.f;
+    for (int v = 0; v < NV; ++v) {
+      Gx[v] = vx ? Gx[v] : 0.f;
+      Gy[v] = vy ? Gy[v] : 0.f;
+    }
+  } else {
+    if (vx) {
+      face2d_weno<NV, HYB>(g, M, fc, c, 0, HYB && smooth_at(smap, c, 0), nv, Gx);
+      face2d_terms(g, P, M, fc, c, 0, Gx);
+    }
+    if (vy) {
+      face2d_weno<NV, HYB>(g, M, fc, c, 1, HYB && smooth_at(smap, c, 1), nv, Gy);
+      face2d_terms(g, P, M, fc, c, 1, Gy);
+    }
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v) sG[ty][tx][v] = Gy[v];

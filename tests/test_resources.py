@@ -14,14 +14,25 @@ pytestmark = pytest.mark.skipif(shutil.which(build.NVCC) is None, reason="nvcc n
 EXTRA = dict(build.UNITS)
 
 
-def _ptxas(unit, tmp):
-    """ptxas -v of a unit: [(mangled kernel name, registers)] and the whole text."""
-    r = subprocess.run([build.NVCC, *build.ARCH, "-O3", "-std=c++17", "--extended-lambda", "-Xptxas", "-v",
-                        *EXTRA[unit], "-I", build.CSRC, "-c", os.path.join(build.CSRC, unit), "-o",
-                        os.path.join(tmp, unit + ".o")], capture_output=True, text=True)
-    assert r.returncode == 0, r.stderr[-2000:]
-    regs = re.findall(r"Compiling entry function '(\w+)'.*?Used (\d+) registers", r.stderr, re.S)
-    return [(name, int(n)) for name, n in regs], r.stderr
+UNITS = ["fst_mixed.cu", "fst_batch.cu", "fst_batch_w16.cu", "fst_batch_w32.cu", "fst_batch_w64.cu"]
+
+
+@pytest.fixture(scope="module")
+def ptxas(tmp_path_factory):
+    """What ptxas -v says of the units: {unit: (its text, [(mangled kernel, registers, bytes spilled)])}."""
+    tmp = str(tmp_path_factory.mktemp("ptxas"))
+
+    def compile(unit):
+        r = subprocess.run([build.NVCC, *build.ARCH, "-O3", "-std=c++17", "--extended-lambda", "-Xptxas", "-v",
+                            *EXTRA[unit], "-I", build.CSRC, "-c", os.path.join(build.CSRC, unit), "-o",
+                            os.path.join(tmp, unit + ".o")], capture_output=True, text=True)
+        assert r.returncode == 0, r.stderr[-2000:]
+        found = re.findall(r"Compiling entry function '(\w+)'.*?(\d+) bytes spill stores.*?Used (\d+) registers",
+                           r.stderr, re.S)
+        return r.stderr, [(name, int(regs), int(spill)) for name, spill, regs in found]
+
+    with ThreadPoolExecutor(len(UNITS)) as ex:
+        return dict(zip(UNITS, ex.map(compile, UNITS)))
 
 
 def _resident(regs, threads):
@@ -29,46 +40,55 @@ def _resident(regs, threads):
     return 65536 // (-(-regs // 8) * 8 * threads) * threads
 
 
-def test_2d_tile_keeps_its_warps(tmp_path):
-    """Both faces' reconstructions side by side raise the tile's registers; the launch
-    bounds hold 1024 threads an SM for every variable count, with learned routing too."""
-    units = ["fst_mixed.cu", "fst_batch_w16.cu", "fst_batch_w32.cu", "fst_batch_w64.cu"]
-    with ThreadPoolExecutor(len(units)) as ex:
-        found = [k for regs, _ in ex.map(lambda u: _ptxas(u, str(tmp_path)), units) for k in regs]
-    seen = 0
-    for name, regs in found:
-        single = re.search(r"k_mrhs2dILi(\d+)ELb[01]E", name)
-        batch = re.search(r"k_brhsILi(\d+)ELi(\d+)ELi(\d+)E", name)
-        if not (single or batch):
-            continue
-        seen += 1
-        threads = 256 if single else int(batch.group(2)) * int(batch.group(3))
+def _tiles(ptxas):
+    """[(kernel, variables, threads a block, registers, bytes spilled)] of the 2D tile."""
+    for _, kernels in ptxas.values():
+        for name, regs, spill in kernels:
+            m = re.search(r"(k_mrhs2d|k_brhs)ILi(\d+)EL([ib])(\d+)EL?i?(\d+)?", name)
+            if m:
+                threads = 256 if m.group(1) == "k_mrhs2d" else int(m.group(4)) * int(m.group(5))
+                yield name, m.group(1) == "k_mrhs2d", int(m.group(2)), threads, regs, spill
+
+
+def test_2d_tile_keeps_its_warps(ptxas):
+    """The launch bounds hold 1024 threads an SM for every variable count, with learned
+    routing too (but for the form of more than 9 variables for grids that need no more than
+    two blocks an SM)."""
+    tiles = [t for t in _tiles(ptxas) if not re.search(r"k_mrhs2dILi20ELb[01]ELi2E", t[0])]
+    assert len(tiles) == 14 + 48  # 7 variable counts with and without routing; 6 counts, 8 shapes
+    for name, _, _, threads, regs, _ in tiles:
         assert _resident(regs, threads) >= 1024, (name, regs)
-    assert seen == 14 + 48  # 7 variable counts with and without routing; 6 counts, 8 shapes
 
 
-def _primitive_passes(tmp):
+def test_2d_tile_of_many_variables_does_not_spill(ptxas):
+    """Both faces' reconstructions side by side need registers that single runs of 7 to 9
+    variables, or with learned routing, do not have: one face after the other there."""
+    for name, single, nv, _, _, spill in _tiles(ptxas):
+        if single and nv <= 9 and (nv >= 7 or "Lb1E" in name):
+            assert spill == 0, (name, spill)
+
+
+def _primitive_passes(ptxas):
     """[(is k_bprim, species or 0 for any number, registers)] of the 2D primitive passes."""
-    out = []
-    for name, regs in _ptxas("fst_batch.cu", tmp)[0] + _ptxas("fst_mixed.cu", tmp)[0]:
-        m = re.search(r"(k_bprimI|k_mprimILi2E)Li(\d+)E", name)
-        if m:
-            out.append((m.group(1) == "k_bprimI", int(m.group(2)), regs))
-    return out
+    for _, kernels in ptxas.values():
+        for name, regs, _ in kernels:
+            m = re.search(r"(k_bprimI|k_mprimILi2E)Li(\d+)E", name)
+            if m:
+                yield m.group(1) == "k_bprimI", int(m.group(2)), regs
 
 
-def test_any_species_primitive_pass_keeps_its_warps(tmp_path):
+def test_any_species_primitive_pass_keeps_its_warps(ptxas):
     """The passes whose species count is not known at compile time: their loops are not
     unrolled 16 times."""
-    found = [(batch, regs) for batch, ns, regs in _primitive_passes(str(tmp_path)) if ns == 0]
+    found = [(batch, regs) for batch, ns, regs in _primitive_passes(ptxas) if ns == 0]
     assert len(found) == 2
     for batch, regs in found:
         assert _resident(regs, 256) >= (768 if batch else 1024), (batch, regs)
 
 
-def test_primitive_passes_keep_their_warps(tmp_path):
+def test_primitive_passes_keep_their_warps(ptxas):
     """The passes of 1 to 5 species."""
-    found = [(batch, ns, regs) for batch, ns, regs in _primitive_passes(str(tmp_path)) if ns > 0]
+    found = [(batch, ns, regs) for batch, ns, regs in _primitive_passes(ptxas) if ns > 0]
     assert len(found) == 10
     for batch, ns, regs in found:
         assert _resident(regs, 256) >= (768 if batch else 1024), (batch, ns, regs)
