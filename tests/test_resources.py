@@ -1,5 +1,5 @@
-"""What ptxas reports for the kernels whose speed hangs on it: registers (warps in
-flight).  Compiles the units here; no GPU."""
+"""What the kernels' speed hangs on and no result shows: the registers and spills that
+ptxas reports, constant memory.  Compiles the units here; no GPU."""
 import os
 import re
 import shutil
@@ -92,3 +92,11 @@ def test_primitive_passes_keep_their_warps(ptxas):
     assert len(found) == 10
     for batch, ns, regs in found:
         assert _resident(regs, 256) >= (768 if batch else 1024), (batch, ns, regs)
+
+
+def test_no_unit_has_constant_memory():
+    """A __constant__ variable costs every launch of every kernel of its unit 0.1 us."""
+    for name in os.listdir(build.CSRC):
+        with open(os.path.join(build.CSRC, name)) as f:
+            code = re.sub(r"//[^\n]*", "", f.read())
+        assert "__constant__" not in code, name
