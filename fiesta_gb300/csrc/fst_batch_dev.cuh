@@ -35,6 +35,10 @@ __device__ __forceinline__ int find_case(const int* __restrict__ off, int n, int
   return lo;
 }
 
+// Part of the key under which the tuner stores a choice: raise it with every change of the
+// tile's code or launch bounds, which the stored times and shapes do not describe.
+constexpr int TILE_VERSION = 2;
+
 // persistent RHS + RK stage over the (case, tile) work list: block b takes
 // work items b, b + gridDim.x, ...; item w is tile w - tile_off[c] of case c
 // (tiles of a case in row-major order, (nci + TXX - 2) / (TXX - 1) per row).
