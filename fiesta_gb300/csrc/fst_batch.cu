@@ -366,7 +366,7 @@ std::string signature(const fst_batch* b) {
   std::ostringstream s;
   s << prop.name << "|cases=" << b->geos.size() << "|cells=" << cells << "|sizes=" << std::hex
     << h << std::dec << "|nv=" << b->nv << "|visc=" << b->cfgs[0].visc
-    << "|ceq=" << b->cfgs[0].ceq << "|tile=" << fstb::TILE_VERSION;
+    << "|ceq=" << b->cfgs[0].ceq << "|buoy=" << b->cfgs[0].buoyancy << "|tile=" << fstb::TILE_VERSION;
   return s.str();
 }
 

@@ -33,3 +33,13 @@ def test_choice_of_another_tile_kernel_is_not_reused(tmp_path):
     assert [e["key"] for e in entries] == [bare, bare + "|tile=1", entry["key"]]  # the others stay
     assert entries[2]["best_ms"] > 1e-6 and entries[2]["candidates"] > 8
     assert shape == tuple(entries[2][k] for k in ("tile_width", "tile_height", "blocks_per_sm"))
+
+
+def test_buoyancy_has_its_own_choice(tmp_path):
+    """The switch adds loads and work to the tile."""
+    cfgs, states = rt_ensemble(ncases=2, nmin=24, nmax=40, seed=3)
+    path = str(tmp_path / "tune.json")
+    assert len(_tuned(cfgs, states, path)[1]) == 1
+    for cfg in cfgs:
+        cfg.buoyancy = 0
+    assert len(_tuned(cfgs, states, path)[1]) == 2
