@@ -19,9 +19,15 @@
 //
 // Measured at 256^3, 9 variables, dx a power of two (per stage): 93.5 ms as one
 // thread per face index with the operators, 49.5 with shared cell terms, fused
-// forms and integer divisions, 25.3 with the products and sums as well, 23.1 with
-// no compare or predicated-off operation left on the FP64 unit (either takes as long
-// as a sum): unit 82 % busy, integer unit 55 %, 44 instructions per FP64 one.
+// forms and integer divisions, 24.3 with the products on the integer pipes, 23.7 with
+// the sums as DFMA, 23.1 with no compare or predicated-off operation left on the FP64
+// unit (either takes as long as a sum): unit 82 % busy, integer unit 55 %, 44
+// instructions per FP64 one.
+// A value outside the range sends the six faces of its line that read it to weno_any,
+// and a warp with such a lane runs both forms.  At 128^3, 9 variables, 3.12 ms: 3.7 with
+// one species falling from 1 to 1e-120 across the box, 3.9 with one at 1e-100 all over,
+// 6.4 with four, 12.0 with every variable in blocks of 16 cells of either kind (both forms
+// on nearly every face); the operators take 13.2 on any of them.
 #pragma once
 #include "fst_internal.h"
 

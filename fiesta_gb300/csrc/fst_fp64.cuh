@@ -204,9 +204,9 @@ FST_HD double eight(double a) { return scale2(a, 3, 8.0); }
 #if defined(__CUDACC__)
 // ---------------------------------------------------------------------------
 // Sums and products as fused operations.  The unit takes a DFMA whose operands
-// are three thread registers every 68 clocks a warp, but a DADD or DMUL, or a
-// DFMA with an immediate, constant or uniform operand, every 81 (GB300, measured
-// on independent chains at 2 to 16 warps per sub-partition).  x 1 + y and x y +
+// are three thread registers every 64 clocks a warp, but a DADD, DMUL or compare
+// every 77 and a DFMA with an immediate, constant or uniform operand every 81 (GB300,
+// every SM busy, independent chains).  x 1 + y and x y +
 // (-0) round exactly as x + y and x y do, zeros' signs included.  lane_const
 // keeps a constant in thread registers: n, a kernel argument that is never
 // negative, makes it look different in every lane.

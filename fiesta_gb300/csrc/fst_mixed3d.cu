@@ -1069,11 +1069,14 @@ inline unsigned cdiv3(long long a, int b) { return (unsigned)((a + b - 1) / b); 
 
 // Planes per block along k for `tiles` (x, y) tiles.  A block costs about three
 // planes of start-up (window loads, first TMA planes, first z face) besides its
-// own, and two blocks fit an SM; the fewest planes x waves wins, the longer march
-// on a tie.  Large grids take KZ3.  Measured per step against KZ3 everywhere:
-// 33x20x18 235 -> 88 us, 61x50x37 244 -> 118, 96x80x64 465 -> 367, 128^3 1229 ->
-// 1206, 160^3 2189 -> 2088, 256^3 the same (fewer planes lose there: 8 planes
-// 2.5 %, 4 planes 9 %).
+// own, and two blocks of the larger kernels fit an SM; the fewest planes x waves wins,
+// the longer march on a tie.  k_mcell3d and the unfused k_mspec3d fit three, but
+// counted so they gain at some sizes what they lose at others (k_mcell3d, 2 species:
+// 100x90x70 20.8 -> 19.0 us, 128^3 35.7 -> 40.7, 200x150x100 50.0 -> 55.0, 192^3 equal;
+// k_mspec3d, 6 species: 96x80x64 58 -> 63, 128^3 217 -> 189, 160^3 348 -> 345).
+// Large grids take KZ3.  Measured per step against KZ3 everywhere (31-column tiles):
+// 33x20x18 235 -> 88 us, 61x50x37 244 -> 118, 96x80x64 465 -> 367, 128^3 1229 -> 1206,
+// 160^3 2189 -> 2088, 256^3 the same (fewer planes lose there: 8 planes 2.5 %, 4 planes 9 %).
 int plan_kz(long long tiles, int nck) {
   const long long slots = 2 * 152;
   int best = KZ3;
